@@ -7,13 +7,15 @@
 //   kernels/finitevolumes/commons/c/commons.cpph:26-67
 //
 // Layout: a patch is (P+2g)^2 cells, row-major [y][x][nData]; patches are
-// stored back to back.  A CTA updates a TX x TY tile of interior cells; the
-// tile and its halo are staged in shared memory, every face flux is
-// computed once per tile, and each cell applies its four face contributions
-// in the reference's order (x faces, then y faces).  The reference also
-// writes the flux contributions of the patch-boundary faces into the first
-// ghost layer of luh_new; that is reproduced.  HBM traffic per cell-update
-// is the state read + write (80 B), halo re-reads excepted.
+// stored back to back.  The tile kernels update a TX x TY tile of interior
+// cells per CTA; the tile and its halo are staged in shared memory, every face
+// flux is computed once per tile, and each cell applies its four face
+// contributions in the reference's order (x faces, then y faces).  The
+// Godunov sweeps (batch, one patch, patch grid) hold a column per lane
+// instead.  The reference also writes the flux contributions of the
+// patch-boundary faces into the first ghost layer of luh_new; the batched
+// updates reproduce that.  HBM traffic per cell-update is the state read +
+// write (80 B), halo re-reads excepted.
 #include <float.h>
 
 #include <cstring>
@@ -302,127 +304,240 @@ __global__ void __launch_bounds__(32 * FVS_WARPS) k_fv_godunov_sweep(FVArgs a) {
   ndt.commit(a, a.next_dt, l == 0);
 }
 
-template <bool PLANAR, bool FUSED, bool GRID = false>
-__device__ __forceinline__ void fv_godunov_tile(const FVArgs& a, int bx, int by, long patch) {
+// Godunov update of a batch of patches (exa_fv_godunov_update) as the same
+// sweep: a warp walks up the rows of one strip of a patch, or, for patches of
+// at most 14 cells, of 32 / (P + 2) whole patches side by side (lane group =
+// patch, lane = column, the outer lanes of a group its ghost columns).  Every
+// cell is read once, every face solved once, x neighbours by shuffle, y
+// neighbours in registers.  The 32 x 8 tile kernel that stands for large
+// single patches leaves most of a tile empty here (10 x 10 patches fill 100
+// of 2 x 256 cells) and re-reads the ghost rows per tile: 40,000 patches of
+// 10 x 10 took it 1259 us and the call 1.29 ms (with a host-made +inf array and
+// a synchronisation for the admissible dt); this way the call takes 0.17 ms,
+// bound by HBM (620 MB: luh once, luh_new in and out).
+// As in the reference, the update is applied to luh_new as it is, and the
+// faces of the patch boundary also reach its first ghost layer: a ghost
+// column belongs to its lane, a ghost row to the lanes above or below it.
+struct FVStrips {
+  long units;    // strips in all: npatches x strips per row x row blocks
+  int width;     // output columns of a strip
+  int per_warp;  // strips side by side in a warp
+  int across, up;  // strips per patch row, row blocks per patch
+  int rows;      // rows of a block
+};
+
+__host__ __device__ inline FVStrips fv_strips(int P, long npatches) {
+  FVStrips s;
+  s.width = P < 30 ? P : 30;
+  s.per_warp = 32 / (s.width + 2);
+  s.across = (P + s.width - 1) / s.width;
+  // whole columns up to 32 rows, blocks of 32 above (two halo rows each)
+  s.rows = P <= 32 ? P : 32;
+  s.up = (P + s.rows - 1) / s.rows;
+  s.units = npatches * s.across * s.up;
+  return s;
+}
+
+template <bool PLANAR>
+__global__ void __launch_bounds__(32 * FVS_WARPS) k_fv_godunov_batch(FVArgs a, FVStrips st) {
+  constexpr int V = kV, C = kV + 1;
+  const int l = threadIdx.x & 31;
+  const int LP = st.width + 2;
+  const int sub = l / LP, c = l - sub * LP;
+  const long warp = (long)blockIdx.x * FVS_WARPS + (threadIdx.x >> 5);
+  const long unit = warp * st.per_warp + sub;
+  const bool live = sub < st.per_warp && unit < st.units;
+  const long patch = live ? unit / (st.across * st.up) : 0;
+  const int part_i = live ? (int)(unit - patch * (st.across * st.up)) : 0;
+  const int sx = part_i % st.across, sy = part_i / st.across;
+  const int S = a.S, D = kV + a.npar, pb = a.g, pe = a.g + a.P;
+  const int k = pb - 1 + sx * st.width + c;
+  const int j0 = pb + sy * st.rows, j1 = j0 + st.rows < pe ? j0 + st.rows : pe;
+  const bool inside = live && c >= 1 && c <= st.width && k < pe;  // an interior column of this strip
+  const bool left_ghost = live && c == 0 && k == pb - 1, right_ghost = live && k == pe;
+  const bool column = live && k <= pe;  // the last strip may be narrower
+  const double* q = a.luh + patch * (long)S * S * D + (column ? k : pb) * D;
+  double* o = a.out + patch * (long)S * S * D + (column ? k : pb) * D;
+  const long row = (long)S * D;
+  const double dt = a.dt_dev ? *a.dt_dev : a.dt;
+  const double cx = dt / a.hx, cy = dt / a.hy;
+  double smx = 0.0, smy = 0.0;
+  double up[V], cyp[C], un[V], part[V];
+  auto load = [&](int j, double* u) {
+#pragma unroll
+    for (int m = 0; m < V; m++) u[m] = q[j * row + m];
+  };
+  load(j0 - 1, up);
+  fv_cell_flux<PLANAR>(up, 1, cyp);
+#pragma unroll
+  for (int m = 0; m < V; m++) part[m] = 0.0;
+  load(j0, un);
+  // (row blocks differ only between the warps of large patches, so the
+  // loop's length is uniform over a warp)
+  for (int j = j0; j <= j1; j++) {
+    double u[V];
+#pragma unroll
+    for (int m = 0; m < V; m++) u[m] = un[m];
+    if (j < j1) load(j + 1, un);
+    double cyr[C], fy[V];
+    fv_cell_flux<PLANAR>(u, 1, cyr);
+    const double sy_ = fv_face_flux(up, u, cyp, cyr, fy);  // the face below row j
+    if (inside) {
+      smy = fmax(smy, sy_);
+      if (j > j0) {
+        double* d = o + (j - 1) * row;
+#pragma unroll
+        for (int m = 0; m < V; m++) d[m] = part[m] - cy * fy[m];
+      }
+      if (j == pb) {
+        double* d = o + (pb - 1) * row;
+#pragma unroll
+        for (int m = 0; m < V; m++) d[m] -= cy * fy[m];
+      }
+      if (j == pe) {
+        double* d = o + pe * row;
+#pragma unroll
+        for (int m = 0; m < V; m++) d[m] += cy * fy[m];
+      }
+    }
+    if (j == j1) break;
+    double v[V];
+    if (inside || left_ghost || right_ghost)
+#pragma unroll
+      for (int m = 0; m < V; m++) v[m] = o[j * row + m];
+    double cxr[C], ul[V], cxl[C], fxl[V], fxr[V];
+    fv_cell_flux<PLANAR>(u, 0, cxr);
+#pragma unroll
+    for (int m = 0; m < V; m++) ul[m] = __shfl_up_sync(0xffffffffu, u[m], 1);
+#pragma unroll
+    for (int m = 0; m < C; m++) cxl[m] = __shfl_up_sync(0xffffffffu, cxr[m], 1);
+    const double sx_ = fv_face_flux(ul, u, cxl, cxr, fxl);
+#pragma unroll
+    for (int m = 0; m < V; m++) fxr[m] = __shfl_down_sync(0xffffffffu, fxl[m], 1);
+    if (inside) {
+#pragma unroll
+      for (int m = 0; m < V; m++) {
+        v[m] += cx * fxl[m];
+        v[m] -= cx * fxr[m];
+        v[m] += cy * fy[m];
+        part[m] = v[m];
+      }
+    } else if (left_ghost) {
+#pragma unroll
+      for (int m = 0; m < V; m++) o[j * row + m] = v[m] - cx * fxr[m];
+    } else if (right_ghost) {
+#pragma unroll
+      for (int m = 0; m < V; m++) o[j * row + m] = v[m] + cx * fxl[m];
+    }
+    // every face of the strip: the left one of each interior cell and, from
+    // the lane right of it, the right one of the strip's last cell
+    if (column && c >= 1) smx = fmax(smx, sx_);
+#pragma unroll
+    for (int m = 0; m < V; m++) up[m] = u[m];
+#pragma unroll
+    for (int m = 0; m < C; m++) cyp[m] = cyr[m];
+  }
+  if (a.max_dt) {
+    // largest bounds of the strip's lanes on its first lane; the division is
+    // monotone, so 0.45 h / max is the minimum of the faces' quotients
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const double x = __shfl_down_sync(0xffffffffu, smx, d), y = __shfl_down_sync(0xffffffffu, smy, d);
+      if (c + d < LP && l + d < 32) {
+        smx = fmax(smx, x);
+        smy = fmax(smy, y);
+      }
+    }
+    if (live && c == 0) {
+      const double v = fmin(DBL_MAX, fmin(0.9 / 2 * a.hx / smx, 0.9 / 2 * a.hy / smy));
+      if (st.across * st.up > 1) atomic_min_pos_double(&a.max_dt[patch], v);
+      else a.max_dt[patch] = v >= 0.0 ? (unsigned long long)__double_as_longlong(v) : 0x7FF0000000000000ULL;
+    }
+  }
+}
+
+// one CTA per small patch (defined with the fused steps below)
+constexpr int FVS_NT = 128;
+constexpr int kFvSmallMax = 16;
+template <bool PLANAR, int SCHEME, bool BATCH>
+__global__ void k_fv_patch_small(FVArgs a);
+inline size_t fv_small_smem(int P, int g, int scheme) {
+  const size_t S = P + 2 * g, R = P + 2;
+  return sizeof(double) * (S * S * kV + (scheme == 1 ? 4 * R * R * kV + 2 * P * (P + 1) * kV
+                                                     : 2 * P * R * (kV + 1)));
+}
+
+// +inf in every slot of a min reduction
+__global__ void k_fv_inf(unsigned long long* slots, long n) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) slots[i] = 0x7FF0000000000000ULL;
+}
+
+template <bool PLANAR, bool GRID = false>
+__device__ __forceinline__ void fv_godunov_tile(const FVArgs& a, int bx, int by) {
   constexpr int V = kV, C = kV + 1;
   constexpr int LX = FV_TX + 2, LY = FV_TY + 2;
   __shared__ double su[LY * LX * V];
   __shared__ double scx[FV_TY * LX * C];  // x: staged rows 1..TY, all columns
   __shared__ double scy[LY * FV_TX * C];  // y: all rows, staged columns 1..TX
-  __shared__ double sred[FV_NT / 32];
-  const int D = V + a.npar, S = a.S, pb = a.g, pe = a.g + a.P;
-  const double* luh = a.luh + patch * (long)S * S * D;
-  double* out = a.out + patch * (long)S * S * D;
-  // FUSED: global cell coordinates of the patch grid (fv_cell_offset)
-  const int k0 = (FUSED ? 0 : pb) + bx * FV_TX, j0 = (FUSED ? 0 : pb) + by * FV_TY;
+  // global cell coordinates of the patch grid (fv_cell_offset)
+  const int k0 = bx * FV_TX, j0 = by * FV_TY;
   const int tid = threadIdx.x;
   for (int i = tid; i < LY * LX; i += FV_NT) {
     const int r = i / LX, c = i % LX;
-    const int j = j0 - 1 + r, k = k0 - 1 + c;
-    if (FUSED) {
-      int flip;
-      const double* q = luh + fv_stencil_offset<GRID>(a, k, j, &flip);
+    int flip;
+    const double* q = a.luh + fv_stencil_offset<GRID>(a, k0 - 1 + c, j0 - 1 + r, &flip);
 #pragma unroll
-      for (int m = 0; m < V; m++) su[i * V + m] = m == flip ? -q[m] : q[m];
-    } else if (j >= 0 && j < S && k >= 0 && k < S) {
-#pragma unroll
-      for (int m = 0; m < V; m++) su[i * V + m] = luh[((long)j * S + k) * D + m];
-    }
+    for (int m = 0; m < V; m++) su[i * V + m] = m == flip ? -q[m] : q[m];
   }
   __syncthreads();
-  // per-cell x fluxes of the cells beside the tile's x faces (rows j < pe,
-  // columns pb-1..pe) and y fluxes of the cells beside its y faces
+  // per-cell x fluxes of the cells beside the tile's x faces and y fluxes of
+  // the cells beside its y faces
   for (int i = tid; i < FV_TY * LX + LY * FV_TX; i += FV_NT) {
     if (i < FV_TY * LX) {
       const int r = i / LX, c = i % LX;
-      const int j = j0 + r, k = k0 - 1 + c;
-      if (FUSED || (j < pe && k <= pe)) fv_cell_flux<PLANAR>(&su[((r + 1) * LX + c) * V], 0, &scx[i * C]);
+      fv_cell_flux<PLANAR>(&su[((r + 1) * LX + c) * V], 0, &scx[i * C]);
     } else {
       const int i2 = i - FV_TY * LX;
       const int r = i2 / FV_TX, c = i2 % FV_TX;
-      const int j = j0 - 1 + r, k = k0 + c;
-      if (FUSED || (j <= pe && k < pe)) fv_cell_flux<PLANAR>(&su[(r * LX + c + 1) * V], 1, &scy[i2 * C]);
+      fv_cell_flux<PLANAR>(&su[(r * LX + c + 1) * V], 1, &scy[i2 * C]);
     }
   }
   __syncthreads();
-  const double dtv = a.dt_dev ? *a.dt_dev : a.dt;
+  const double dtv = *a.dt_dev;
   const double cx = dtv / a.hx, cy = dtv / a.hy;
-  double dtl = DBL_MAX;
   FVNextDt ndt;
-  {
-    const int r = tid / FV_TX, c = tid % FV_TX;
-    const int j = j0 + r, k = k0 + c;
-    const bool valid = FUSED ? (j < a.P * a.npy && k < a.P * a.npx) : (j < pe && k < pe);
+  const int r = tid / FV_TX, c = tid % FV_TX;
+  const int j = j0 + r, k = k0 + c;
+  const bool valid = j < a.P * a.npy && k < a.P * a.npx;
+  // output cell, addressed before the face fluxes hold their registers
+  double* o = a.out + (valid ? fv_cell_offset<GRID>(a, k, j) : 0);
+  if (valid) {
     double fxl[V], fxr[V], fyb[V], fyt[V];
-    // output cell, addressed before the face fluxes hold their registers
-    double* o = FUSED ? a.out + (valid ? fv_cell_offset<GRID>(a, k, j) : 0) : out + ((long)j * S + k) * D;
-    if (valid) {
-      const double* q = &su[((r + 1) * LX + c + 1) * V];
-      const double sxl = fv_face_flux(q - V, q, &scx[(r * LX + c) * C], &scx[(r * LX + c + 1) * C], fxl);
-      const double sxr = fv_face_flux(q, q + V, &scx[(r * LX + c + 1) * C], &scx[(r * LX + c + 2) * C], fxr);
-      const double syb = fv_face_flux(q - LX * V, q, &scy[(r * FV_TX + c) * C], &scy[((r + 1) * FV_TX + c) * C], fyb);
-      const double syt = fv_face_flux(q, q + LX * V, &scy[((r + 1) * FV_TX + c) * C], &scy[((r + 2) * FV_TX + c) * C], fyt);
-      if (!FUSED && a.max_dt) {
-        // min over faces of 0.45 h / s = 0.45 h / (max over faces of s):
-        // the division is monotone, so the same value as per face
-        dtl = fmin(0.9 / 2 * a.hx / fmax(sxl, sxr), 0.9 / 2 * a.hy / fmax(syb, syt));
-      }
-      double un[V];
+    const double* q = &su[((r + 1) * LX + c + 1) * V];
+    fv_face_flux(q - V, q, &scx[(r * LX + c) * C], &scx[(r * LX + c + 1) * C], fxl);
+    fv_face_flux(q, q + V, &scx[(r * LX + c + 1) * C], &scx[(r * LX + c + 2) * C], fxr);
+    fv_face_flux(q - LX * V, q, &scy[(r * FV_TX + c) * C], &scy[((r + 1) * FV_TX + c) * C], fyb);
+    fv_face_flux(q, q + LX * V, &scy[((r + 1) * FV_TX + c) * C], &scy[((r + 2) * FV_TX + c) * C], fyt);
+    double un[V];
 #pragma unroll
-      for (int m = 0; m < V; m++) {
-        double u = FUSED ? q[m] : o[m];
-        u += cx * fxl[m];
-        u -= cx * fxr[m];
-        u += cy * fyb[m];
-        u -= cy * fyt[m];
-        o[m] = u;
-        un[m] = u;
-      }
-      if (FUSED) {
-        ndt.add<PLANAR>(un);
-      }
+    for (int m = 0; m < V; m++) {
+      double u = q[m];
+      u += cx * fxl[m];
+      u -= cx * fxr[m];
+      u += cy * fyb[m];
+      u -= cy * fyt[m];
+      o[m] = u;
+      un[m] = u;
     }
-    if (FUSED) {
-      ndt.commit(a, a.next_dt, (tid & 31) == 0);
-      return;
-    }
-    // first ghost layer, as the reference's face loops touch it
-    if (valid && k0 == pb && c == 0) {
-      o = out + ((long)j * S + (pb - 1)) * D;
-#pragma unroll
-      for (int m = 0; m < V; m++) o[m] -= cx * fxl[m];
-    }
-    if (valid && k == pe - 1) {
-      double* o = out + ((long)j * S + pe) * D;
-#pragma unroll
-      for (int m = 0; m < V; m++) o[m] += cx * fxr[m];
-    }
-    if (valid && j0 == pb && r == 0) {
-      double* o = out + ((long)(pb - 1) * S + k) * D;
-#pragma unroll
-      for (int m = 0; m < V; m++) o[m] -= cy * fyb[m];
-    }
-    if (valid && j == pe - 1) {
-      double* o = out + ((long)pe * S + k) * D;
-#pragma unroll
-      for (int m = 0; m < V; m++) o[m] += cy * fyt[m];
-    }
+    ndt.add<PLANAR>(un);
   }
-  if (a.max_dt) {
-    for (int o = 16; o > 0; o >>= 1) dtl = fmin(dtl, __shfl_xor_sync(0xffffffffu, dtl, o));
-    if ((tid & 31) == 0) sred[tid >> 5] = dtl;
-    __syncthreads();
-    if (tid == 0) {
-      double m = sred[0];
-      for (int w = 1; w < FV_NT / 32; w++) m = fmin(m, sred[w]);
-      atomic_min_pos_double(&a.max_dt[patch], m);
-    }
-  }
+  ndt.commit(a, a.next_dt, (tid & 31) == 0);
 }
 
-template <bool PLANAR, bool FUSED, bool GRID = false>
+template <bool PLANAR, bool GRID = false>
 __global__ void __launch_bounds__(FV_NT, 5) k_fv_godunov(FVArgs a) {
-  fv_godunov_tile<PLANAR, FUSED, GRID>(a, blockIdx.x, blockIdx.y, blockIdx.z);
+  fv_godunov_tile<PLANAR, GRID>(a, blockIdx.x, blockIdx.y);
 }
 
 // -------------------------------------------------------- MUSCL-Hancock
@@ -1012,7 +1127,7 @@ __global__ void __launch_bounds__(FV_NT, 5) k_fv_godunov_serve(const FVServePatc
   const FVServePatch& p = pt[fv_serve_find(pt, np, blockIdx.x)];
   const FVArgs a = fv_serve_args(p);
   const int t = blockIdx.x - p.tile0;
-  fv_godunov_tile<PLANAR, true>(a, t % p.tiles_x, t / p.tiles_x, 0);
+  fv_godunov_tile<PLANAR>(a, t % p.tiles_x, t / p.tiles_x);
 }
 
 // per patch: time += dt, dt = next dt, next dt = +inf, state buffer flipped
@@ -1135,13 +1250,13 @@ exa_status_t fv_patch_step_async(int scheme, const exa_fv_desc_t& d, const doubl
   const bool planar = d.pde == EXA_PDE_EULER_PLANAR;
   dim3 grid((d.patch + FVP_TX - 1) / FVP_TX, (d.patch + FVP_TY - 1) / FVP_TY, 1);
   if (scheme == 0) {
-    // shared face fluxes per tile (k_fv_godunov<..., FUSED>): measured faster
+    // shared face fluxes per tile (k_fv_godunov): measured faster
     // for first order than per-cell face fluxes (k_fv_godunov_periodic),
     // whose doubled Riemann work is not paid back by the saved barrier
     dim3 gt((d.patch + FV_TX - 1) / FV_TX, (d.patch + FV_TY - 1) / FV_TY, 1);
     static bool gattr[2] = {false, false};
     if (!gattr[planar]) {
-      cudaError_t e = cudaFuncSetAttribute(planar ? k_fv_godunov<true, true> : k_fv_godunov<false, true>,
+      cudaError_t e = cudaFuncSetAttribute(planar ? k_fv_godunov<true> : k_fv_godunov<false>,
                                            cudaFuncAttributePreferredSharedMemoryCarveout,
                                            (int)cudaSharedmemCarveoutMaxShared);
       if (e != cudaSuccess) return cuda_status(e, "godunov attribute");
@@ -1153,9 +1268,9 @@ exa_status_t fv_patch_step_async(int scheme, const exa_fv_desc_t& d, const doubl
       if (planar) k_fv_godunov_sweep<true, false><<<gs, 32 * FVS_WARPS, 0, st>>>(a);
       else k_fv_godunov_sweep<false, false><<<gs, 32 * FVS_WARPS, 0, st>>>(a);
     } else if (planar) {
-      k_fv_godunov<true, true><<<gt, FV_NT, 0, st>>>(a);
+      k_fv_godunov<true><<<gt, FV_NT, 0, st>>>(a);
     } else {
-      k_fv_godunov<false, true><<<gt, FV_NT, 0, st>>>(a);
+      k_fv_godunov<false><<<gt, FV_NT, 0, st>>>(a);
     }
   } else {
     static bool attr[2] = {false, false};
@@ -1219,13 +1334,15 @@ static exa_status_t fv_update(int scheme, const exa_fv_desc_t* desc, long npatch
   if (npatches == 0) return EXA_OK;
   if (npatches > 65535) return set_error(EXA_EINVAL, "at most 65535 patches per call");
   cudaStream_t st = as_stream(stream);
+  // +inf before the minima, in stream order
+  auto clear_max_dt = [&]() -> exa_status_t {
+    if (!max_dt) return EXA_OK;
+    k_fv_inf<<<(unsigned)((npatches + 255) / 256), 256, 0, st>>>((unsigned long long*)max_dt, npatches);
+    count_launch();
+    return cuda_status(cudaGetLastError(), "k_fv_inf");
+  };
   if (desc->dim == 3) {
-    if (max_dt) {
-      std::vector<unsigned long long> inf(npatches, 0x7FF0000000000000ULL);
-      cudaError_t e = cudaMemcpyAsync(max_dt, inf.data(), 8 * npatches, cudaMemcpyHostToDevice, st);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-      if (e != cudaSuccess) return cuda_status(e, "max_dt init");
-    }
+    if (exa_status_t s = clear_max_dt()) return s;
     const double h[3] = {desc->dx[0] / desc->patch, desc->dx[1] / desc->patch, desc->dx[2] / desc->patch};
     return fv3_update(scheme, desc->patch, desc->ghost, desc->nvar + desc->npar, h, npatches, luh_new, luh, dt,
                       nullptr, max_dt, nullptr, nullptr, st);
@@ -1235,31 +1352,43 @@ static exa_status_t fv_update(int scheme, const exa_fv_desc_t* desc, long npatch
   a.luh = luh;
   a.out = luh_new;
   a.max_dt = (unsigned long long*)max_dt;
-  if (max_dt) {
-    // +inf bit pattern 0x7FF0000000000000 = bytes 00..00 F0 7F
-    std::vector<unsigned long long> inf(npatches, 0x7FF0000000000000ULL);
-    cudaError_t e = cudaMemcpyAsync(max_dt, inf.data(), 8 * npatches, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return cuda_status(e, "max_dt init");
-  }
-  dim3 grid((desc->patch + FV_TX - 1) / FV_TX, (desc->patch + FV_TY - 1) / FV_TY, (unsigned)npatches);
   const bool planar = desc->pde == EXA_PDE_EULER_PLANAR;
   if (scheme == 0) {
-    if (planar) k_fv_godunov<true, false><<<grid, FV_NT, 0, st>>>(a);
-    else k_fv_godunov<false, false><<<grid, FV_NT, 0, st>>>(a);
-  } else {
-    static bool attr[2] = {false, false};
-    if (!attr[planar]) {
-      cudaError_t e = planar ? cudaFuncSetAttribute(k_fv_muscl<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMusclSmem)
-                             : cudaFuncSetAttribute(k_fv_muscl<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMusclSmem);
-      if (e != cudaSuccess) return cuda_status(e, "muscl attribute");
-      attr[planar] = true;
-    }
-    if (planar) k_fv_muscl<true, false><<<grid, FV_NT, kMusclSmem, st>>>(a);
-    else k_fv_muscl<false, false><<<grid, FV_NT, kMusclSmem, st>>>(a);
+    const FVStrips s = fv_strips(desc->patch, npatches);
+    if (s.across * s.up > 1)
+      if (exa_status_t e = clear_max_dt()) return e;
+    const long warps = (s.units + s.per_warp - 1) / s.per_warp;
+    const long blocks = (warps + FVS_WARPS - 1) / FVS_WARPS;
+    if (blocks > 0x7fffffffL) return set_error(EXA_EINVAL, "too many cells");
+    if (planar) k_fv_godunov_batch<true><<<(unsigned)blocks, 32 * FVS_WARPS, 0, st>>>(a, s);
+    else k_fv_godunov_batch<false><<<(unsigned)blocks, 32 * FVS_WARPS, 0, st>>>(a, s);
+    count_launch();
+    return cuda_status(cudaGetLastError(), "k_fv_godunov_batch");
   }
+  if (exa_status_t s = clear_max_dt()) return s;
+  if (desc->patch <= kFvSmallMax) {
+    auto kern = planar ? k_fv_patch_small<true, 1, true> : k_fv_patch_small<false, 1, true>;
+    const size_t smem = fv_small_smem(desc->patch, desc->ghost, 1);
+    if (smem <= 200 * 1024) {
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return cuda_status(e, "muscl batch attribute");
+      kern<<<(unsigned)npatches, FVS_NT, smem, st>>>(a);
+      count_launch();
+      return cuda_status(cudaGetLastError(), "k_fv_patch_small");
+    }
+  }
+  dim3 grid((desc->patch + FV_TX - 1) / FV_TX, (desc->patch + FV_TY - 1) / FV_TY, (unsigned)npatches);
+  static bool attr[2] = {false, false};
+  if (!attr[planar]) {
+    cudaError_t e = planar ? cudaFuncSetAttribute(k_fv_muscl<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMusclSmem)
+                           : cudaFuncSetAttribute(k_fv_muscl<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMusclSmem);
+    if (e != cudaSuccess) return cuda_status(e, "muscl attribute");
+    attr[planar] = true;
+  }
+  if (planar) k_fv_muscl<true, false><<<grid, FV_NT, kMusclSmem, st>>>(a);
+  else k_fv_muscl<false, false><<<grid, FV_NT, kMusclSmem, st>>>(a);
   count_launch();
-  return cuda_status(cudaGetLastError(), scheme == 0 ? "k_fv_godunov" : "k_fv_muscl");
+  return cuda_status(cudaGetLastError(), "k_fv_muscl");
 }
 
 exa_status_t exa_fv_godunov_update(const exa_fv_desc_t* desc, long npatches, double* luh_new,
@@ -1528,10 +1657,11 @@ namespace exa {
 // own four face fluxes, applies them in the reference's order and writes
 // only the interior of the output; the new state's CFL dt is reduced in the
 // same pass.  Same arithmetic per cell as the tile kernels.
-constexpr int FVS_NT = 128;
-constexpr int kFvSmallMax = 16;
-
-template <bool PLANAR, int SCHEME>
+//
+// BATCH (exa_fv_musclhancock_update): as the reference's per-patch update
+// instead, luh_new += face contributions, also in its first ghost layer, and
+// the admissible dt per patch.
+template <bool PLANAR, int SCHEME, bool BATCH>
 __global__ void __launch_bounds__(FVS_NT) k_fv_patch_small(FVArgs a) {
   constexpr int V = kV;
   extern __shared__ double sm[];
@@ -1558,11 +1688,16 @@ __global__ void __launch_bounds__(FVS_NT) k_fv_patch_small(FVArgs a) {
     const double* luh = a.luh + patch * (long)S * S * D;
     double* out = a.out + patch * (long)S * S * D;
     const int tid = threadIdx.x;
-    const double hx = a.hx, hy = a.hy, dt = *a.dt_dev;
+    const double hx = a.hx, hy = a.hy, dt = BATCH && !a.dt_dev ? a.dt : *a.dt_dev;
     // reciprocal cell sizes: multiplications instead of the reference's
     // divisions (an FP64 division is a long dependent chain)
     const double ihx = 1.0 / hx, ihy = 1.0 / hy;
-    for (int i = tid; i < S * S * V; i += FVS_NT) su[i] = luh[i];  // D == V: no parameters here
+    if (!BATCH || a.npar == 0) {
+      for (int i = tid; i < S * S * V; i += FVS_NT) su[i] = luh[i];
+    } else {
+      for (int i = tid; i < S * S * V; i += FVS_NT) su[i] = luh[(i / V) * D + i % V];
+    }
+    double dtl = DBL_MAX;  // BATCH: admissible dt over this thread's faces
     __syncthreads();
     if (SCHEME == 1) {
       for (int i = tid; i < R * R; i += FVS_NT) {
@@ -1629,12 +1764,14 @@ __global__ void __launch_bounds__(FVS_NT) k_fv_patch_small(FVArgs a) {
         if (i < P * (P + 1)) {
           const int r = i / (P + 1), c = i % (P + 1);  // face left of column pb + c, row pb + r
           const int ic = (r + 1) * R + c + 1;
-          rusanov<PLANAR>(&wRx[(ic - 1) * V], &wLx[ic * V], 0, &sfx[i * V]);
+          const double s = rusanov<PLANAR>(&wRx[(ic - 1) * V], &wLx[ic * V], 0, &sfx[i * V]);
+          if (BATCH) dtl = fmin(dtl, 0.99 / 2 * hx / s);
         } else {
           const int i2 = i - P * (P + 1);
           const int r = i2 / P, c = i2 % P;  // face below row pb + r, column pb + c
           const int ic = (r + 1) * R + c + 1;
-          rusanov<PLANAR>(&wRy[(ic - R) * V], &wLy[ic * V], 1, &sfy[i2 * V]);
+          const double s = rusanov<PLANAR>(&wRy[(ic - R) * V], &wLy[ic * V], 1, &sfy[i2 * V]);
+          if (BATCH) dtl = fmin(dtl, 0.99 / 2 * hy / s);
         }
       }
       __syncthreads();
@@ -1675,18 +1812,31 @@ __global__ void __launch_bounds__(FVS_NT) k_fv_patch_small(FVArgs a) {
           fyt[m] = sfy[((r + 1) * P + c) * V + m];
         }
       }
-      fv_update_store_dt<PLANAR>(a, out + ((long)j * S + k) * D, U, fxl, fxr, fyb, fyt, cx, cy, dtn);
+      if constexpr (BATCH) {
+        double* o = out + ((long)j * S + k) * D;
+#pragma unroll
+        for (int m = 0; m < V; m++) {
+          double u = o[m];
+          u += cx * fxl[m];
+          u -= cx * fxr[m];
+          u += cy * fyb[m];
+          u -= cy * fyt[m];
+          o[m] = u;
+          if (c == 0) o[m - D] -= cx * fxl[m];
+          if (c == P - 1) o[m + D] += cx * fxr[m];
+          if (r == 0) o[m - (long)S * D] -= cy * fyb[m];
+          if (r == P - 1) o[m + (long)S * D] += cy * fyt[m];
+        }
+      } else {
+        fv_update_store_dt<PLANAR>(a, out + ((long)j * S + k) * D, U, fxl, fxr, fyb, fyt, cx, cy, dtn);
+      }
     }
+    if (BATCH) dtn = dtl;
     for (int o = 16; o > 0; o >>= 1) dtn = fmin(dtn, __shfl_xor_sync(0xffffffffu, dtn, o));
-    if ((tid & 31) == 0 && a.next_dt) atomic_min_pos_double(a.next_dt, dtn);
+    unsigned long long* slot = BATCH ? (a.max_dt ? a.max_dt + patch : nullptr) : a.next_dt;
+    if ((tid & 31) == 0 && slot) atomic_min_pos_double(slot, dtn);
     __syncthreads();
   }
-}
-
-inline size_t fv_small_smem(int P, int g, int scheme) {
-  const size_t S = P + 2 * g, R = P + 2;
-  return sizeof(double) * (S * S * kV + (scheme == 1 ? 4 * R * R * kV + 2 * P * (P + 1) * kV
-                                                     : 2 * P * R * (kV + 1)));
 }
 
 // Subcell patches of the limiting ADER-DG grid: patch `cell` of a periodic
@@ -1756,8 +1906,8 @@ exa_status_t fv_subcell_step(int scheme, int planar, int P, int g, int npx, int 
   a.list = list;
   a.count = count;
   const size_t smem = fv_small_smem(P, g, scheme);
-  auto kern = scheme == 0 ? (planar ? k_fv_patch_small<true, 0> : k_fv_patch_small<false, 0>)
-                          : (planar ? k_fv_patch_small<true, 1> : k_fv_patch_small<false, 1>);
+  auto kern = scheme == 0 ? (planar ? k_fv_patch_small<true, 0, false> : k_fv_patch_small<false, 0, false>)
+                          : (planar ? k_fv_patch_small<true, 1, false> : k_fv_patch_small<false, 1, false>);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return cuda_status(e, "subcell FV attribute");
   const long grid = maxcells < 16L * sms ? maxcells : 16L * sms;  // CTAs loop over the listed patches
@@ -1832,7 +1982,7 @@ static exa_status_t fv_patchgrid_step_one(exa_fv_patchgrid* g) {
   if (g->scheme == 0) {
     static bool gattr[2] = {false, false};
     if (!gattr[planar]) {
-      cudaError_t e = cudaFuncSetAttribute(planar ? k_fv_godunov<true, true, true> : k_fv_godunov<false, true, true>,
+      cudaError_t e = cudaFuncSetAttribute(planar ? k_fv_godunov<true, true> : k_fv_godunov<false, true>,
                                            cudaFuncAttributePreferredSharedMemoryCarveout,
                                            (int)cudaSharedmemCarveoutMaxShared);
       if (e != cudaSuccess) return cuda_status(e, "godunov attribute");
@@ -1845,8 +1995,8 @@ static exa_status_t fv_patchgrid_step_one(exa_fv_patchgrid* g) {
       else k_fv_godunov_sweep<false, true><<<gs, 32 * FVS_WARPS, 0, g->st>>>(a);
     } else {
       const dim3 grid((unsigned)((NX + FV_TX - 1) / FV_TX), (unsigned)((NY + FV_TY - 1) / FV_TY), 1);
-      if (planar) k_fv_godunov<true, true, true><<<grid, FV_NT, 0, g->st>>>(a);
-      else k_fv_godunov<false, true, true><<<grid, FV_NT, 0, g->st>>>(a);
+      if (planar) k_fv_godunov<true, true><<<grid, FV_NT, 0, g->st>>>(a);
+      else k_fv_godunov<false, true><<<grid, FV_NT, 0, g->st>>>(a);
     }
   } else {
     static bool attr[2] = {false, false};
