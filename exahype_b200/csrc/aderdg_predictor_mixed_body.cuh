@@ -156,14 +156,14 @@ __device__ __forceinline__ void mixed_base_derivative(const PredArgs& a, const d
 // (the reference's formulas, FP64).
 //
 // Both are contractions along lines, so they run as line tasks (direction
-// d, line c, variable m; the same numbering as the line-owner predictor):
-// a task reads the B values of Qh and Fh_d on its line once and produces
-// the two face values of that line (the face node of line c is c) and the
-// B line sums  sum_p Kxi[i][p] Fh_d[p]  of the volume integral, which the
-// node threads weight and sum over directions.  sD: the cell's FP64 staging
+// d, line c, variable m; variable fastest, so a warp stores whole 32-byte
+// sectors of the faces): a task reads the B values of Qh and Fh_d on its
+// line once and produces the two face values of that line (the face node of
+// line c is c) and the B weighted line sums of the volume integral, which
+// are then summed over directions in memory order, coalesced.  sD: the cell's FP64 staging
 // area, MixShape::STAGE_D doubles: Qh [NPC][V], Fh [DIM][NPC][V],
 // volume-integral line sums [DIM][NPC][V].
-template <int DIM, int N>
+template <int DIM, int N, int G = MixShape<DIM, N>::G>
 __device__ __forceinline__ void dg_line_outputs(const PredArgs& a, long cell, int s, bool valid, bool active,
                                                 double* sD, int it, bool conv);
 
@@ -203,13 +203,13 @@ __device__ __forceinline__ void mixed_outputs(const PredArgs& a, long cell, int 
 
 // Face extrapolations and volume integral of a predictor cell from the
 // FP64 staging area written by the caller (Qh [NPC][V], Fh [DIM][NPC][V];
-// every thread of the CTA calls it after the caller's stores): see
-// mixed_outputs.
-template <int DIM, int N>
+// every thread of the CTA calls it after the caller's stores; G threads per
+// cell): see mixed_outputs.
+template <int DIM, int N, int G>
 __device__ __forceinline__ void dg_line_outputs(const PredArgs& a, long cell, int s, bool valid, bool active,
                                                 double* sD, int it, bool conv) {
   using S = MixShape<DIM, N>;
-  constexpr int B = S::B, V = S::V, NPC = S::NPC, G = S::G, NF = S::NF;
+  constexpr int B = S::B, V = S::V, NPC = S::NPC, NF = S::NF;
   constexpr int L = NPC / B, TPD = L * V, TPT = (TPD + G - 1) / G;
   const DGConst& T = c_dg[N];
   double* sQh = sD;                     // [NPC][V]
@@ -223,7 +223,9 @@ __device__ __forceinline__ void dg_line_outputs(const PredArgs& a, long cell, in
     for (int r = 0; r < TPT; r++) {
       const int k = s + r * G;
       if (k >= TPD) continue;
-      const int c = k % L, m = k / L;
+      const int c = k / V, m = k - c * V;
+      // weights of the line's two (one) other coordinates
+      const double wc = DIM == 3 ? T.w[c / B] * T.w[c % B] : T.w[c];
 #pragma unroll
       for (int d = 0; d < DIM; d++) {
         double q[B], f[B];
@@ -242,45 +244,34 @@ __device__ __forceinline__ void dg_line_outputs(const PredArgs& a, long cell, in
           fl += f[p] * T.fl[p];
           fr += f[p] * T.fr[p];
         }
-        qb[((2 * d) * NF + c) * V + m] = ql;
-        qb[((2 * d + 1) * NF + c) * V + m] = qr;
-        fb[((2 * d) * NF + c) * V + m] = fl;
-        fb[((2 * d + 1) * NF + c) * V + m] = fr;
+        qb[(2 * d) * NF * V + k] = ql;
+        qb[(2 * d + 1) * NF * V + k] = qr;
+        fb[(2 * d) * NF * V + k] = fl;
+        fb[(2 * d + 1) * NF * V + k] = fr;
         // volume-integral line sums
+        const double us = a.idx[d] * wc;
 #pragma unroll
         for (int i = 0; i < B; i++) {
           double v = 0.0;
 #pragma unroll
           for (int p = 0; p < B; p++) v += T.kxi[i][p] * f[p];
           const int node = d == 0 ? line_node<B, 0>(c, i) : (d == 1 ? line_node<B, 1>(c, i) : line_node<B, 2>(c, i));
-          sVI[(d * NPC + node) * V + m] = v;
+          sVI[(d * NPC + node) * V + m] = v * us;
         }
       }
     }
   }
   __syncthreads();
   if (!valid) return;
-  if (active) {
-    // lduh[s] = sum_d (idx_d prod_{e != d} w[s_e]) sum_p Kxi[s_d][p] Fh_d(s_d -> p)
-    int sd[3];
-    sd[0] = s % B;
-    sd[1] = (s / B) % B;
-    sd[2] = DIM == 3 ? s / (B * B) : 0;
+  {
+    // lduh[node] = sum_d (idx_d prod_{e != d} w[s_e]) sum_p Kxi[s_d][p] Fh_d(s_d -> p)
     double* lduh = a.lduh + cell * (long)NPC * V;
-    double out[V];
+    for (int k = s; k < NPC * V; k += G) {
+      double out = sVI[k];
 #pragma unroll
-    for (int m = 0; m < V; m++) out[m] = 0.0;
-#pragma unroll
-    for (int d = 0; d < DIM; d++) {
-      double us = a.idx[d];
-#pragma unroll
-      for (int e = 0; e < DIM; e++)
-        if (e != d) us *= T.w[sd[e]];
-#pragma unroll
-      for (int m = 0; m < V; m++) out[m] += sVI[(d * NPC + s) * V + m] * us;
+      for (int d = 1; d < DIM; d++) out += sVI[d * NPC * V + k];
+      lduh[k] = out;
     }
-#pragma unroll
-    for (int m = 0; m < V; m++) lduh[s * V + m] = out[m];
   }
   if (s == 0) {
     if (a.iters) a.iters[cell] = it;
