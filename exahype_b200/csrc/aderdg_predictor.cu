@@ -28,6 +28,7 @@
 #include "aderdg_predictor_body.cuh"
 #include "aderdg_predictor_fp64_lines_body.cuh"
 #include "aderdg_predictor_fp64_prog_body.cuh"
+#include "aderdg_predictor_pencil_body.cuh"
 
 namespace exa {
 
@@ -118,25 +119,73 @@ static exa_status_t launch_prog_fp64(const PredArgs& a, cudaStream_t st) {
   return cuda_status(cudaGetLastError(), "k_predictor_prog launch");
 }
 
+// space-time pencil form (aderdg_predictor_pencil_body.cuh)
+// resident CTAs the registers are bounded for (measured; one step down
+// spills, one up leaves the SM emptier): 2D 96 / 128 / 168 / 168 registers
+// for orders 2..5, 3D 200 / 168 / 255 for orders 3..5
+template <int DIM, int N>
+constexpr int pencil_minb() {
+  return DIM == 3 ? (N == 3 ? 5 : (N == 4 ? 3 : 1)) : (N == 2 ? 5 : (N == 3 ? 4 : (N == 4 ? 3 : 2)));
+}
+
+template <int DIM, int N, bool PLANAR>
+__global__ void __launch_bounds__(PencilShape<DIM, N>::NT, pencil_minb<DIM, N>()) k_predictor_pencil(PredArgs a) {
+  extern __shared__ double smem[];
+  predictor_pencil_block<DIM, N, PLANAR>(a, blockIdx.x, smem);
+}
+
+template <int DIM, int N, bool PLANAR>
+static exa_status_t launch_pencil(const PredArgs& a, cudaStream_t st) {
+  using S = PencilShape<DIM, N>;
+  auto kern = k_predictor_pencil<DIM, N, PLANAR>;
+  const size_t smem = sizeof(double) * S::SM_DOUBLES;
+  static bool attr_done[64] = {false};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!attr_done[dev & 63]) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
+                               (int)cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return cuda_status(e, "predictor (pencil) attribute");
+    attr_done[dev & 63] = true;
+  }
+  if (a.ncells <= 0) return EXA_OK;
+  const long blocks = (a.ncells + S::CPB - 1) / S::CPB;
+  if (blocks > 0x7fffffffL) return set_error(EXA_EINVAL, "too many cells");
+  kern<<<(unsigned)blocks, S::NT, smem, st>>>(a);
+  count_launch();
+  return cuda_status(cudaGetLastError(), "k_predictor_pencil launch");
+}
+
 template <int DIM, int N>
 static exa_status_t launch_dn(const exa_aderdg_desc_t& d, const PredArgs& a, int full,
                               cudaStream_t st) {
   const bool planar = d.pde == EXA_PDE_EULER_PLANAR;
-  // knob 3: 1 = node-gather, 2 = line-owner contraction, 3 = the
-  // progressive line-owner form (FP64, not for the reference-temporaries
-  // mode); default: progressive for order 4 (3D Euler: 3 CTAs per SM, it
-  // measured 6.5 % faster than the line-owner kernel at 81^3; 2D: 7 % in
-  // the ensemble's order-4 launches), line-owner for the other orders >= 4,
-  // where it measured faster in 2D and 3D (for orders 2-3 the cell has more
-  // line tasks than threads and node-gather wins)
+  // Default: the pencil form, except 3D order 2.  us per call, pencil against
+  // the faster of the other forms (node-gather, line-owner, progressive
+  // line-owner): 2D orders 2..5 308 / 478, 396 / 524, 541 / 721, 566 / 845
+  // (156,000 to 27,641 cells), 3D orders 3..5 1780 / 2253, 3333 / 4073,
+  // 2365 / 2823 (82,000, 68,921 and 15,000 cells).  In 3D order 2 (27 threads
+  // a cell, 45 T tasks on them) it measured 1794 against 1757 for line-owner.
+  // knob 3 selects another: 1 = node-gather, 2 = line-owner contraction, 3 =
+  // the progressive line-owner form (order 4; others line-owner).  Node-gather
+  // also serves the reference-temporaries mode and parameters.
   const int variant = tune_get(kTuneFp64Variant, 0);
+  if constexpr (!(DIM == 3 && N == 2))
+    if (d.npar == 0 && !full && variant == 0) {
+      if constexpr (DIM == 2)
+        if (planar) return launch_pencil<DIM, N, true>(a, st);
+      if (planar) return set_error(EXA_EINVAL, "planar Euler is a 2D PDE");
+      return launch_pencil<DIM, N, false>(a, st);
+    }
   if constexpr (N == 4)
-    if (d.npar == 0 && !full && (variant == 3 || variant == 0) && !(DIM == 3 && planar)) {
+    if (d.npar == 0 && !full && variant == 3 && !(DIM == 3 && planar)) {
       if constexpr (DIM == 2)
         if (planar) return launch_prog_fp64<DIM, N, true>(a, st);
       return launch_prog_fp64<DIM, N, false>(a, st);
     }
-  if (d.npar == 0 && !full && (variant >= 2 || (variant == 0 && N >= 4))) {
+  if (d.npar == 0 && !full && (variant >= 2 || variant == 0)) {
     if (DIM == 3 && planar) return set_error(EXA_EINVAL, "planar Euler is a 2D PDE");
     return planar ? launch_lines_fp64<DIM, N, true>(a, st) : launch_lines_fp64<DIM, N, false>(a, st);
   }

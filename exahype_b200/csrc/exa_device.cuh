@@ -22,6 +22,7 @@ struct DGConst {
   double deriv[10][10]; // Kxi[p][l] / w_l  -> derivative onto node l
   double tA[10][10];    // iK1[t][n] * w_n  (Picard time contraction)
   double c0[10];        // sum_n iK1[t][n] F0[n]
+  double tAsum[10];     // sum_n tA[t][n] (slices that all hold the same value)
   double fl[10];        // FLCoeff
   double fr[10];        // FRCoeff
   double pnpm;          // CFL safety factor of order N

@@ -24,6 +24,7 @@ static void build() {
       T.fl[i] = exa_flcoeff[N][i];
       T.fr[i] = exa_frcoeff[N][i];
       T.c0[i] = 0.0;
+      T.tAsum[i] = 0.0;
       for (int j = 0; j < 10; j++) {
         T.kxi[i][j] = exa_kxi[N][i][j];
         T.deriv[i][j] = 0.0;
@@ -37,6 +38,7 @@ static void build() {
       for (int n = 0; n < B; n++) {
         T.tA[t][n] = exa_ik1[N][t][n] * exa_gl_weights[N][n];
         c += exa_ik1[N][t][n] * exa_f0[N][n];
+        T.tAsum[t] += T.tA[t][n];
       }
       T.c0[t] = c;
     }
