@@ -26,8 +26,7 @@
 #include "aderdg_predictor_body.cuh"
 #include "aderdg_predictor_mixed_body.cuh"
 #include "aderdg_predictor_lines_body.cuh"
-#include "aderdg_predictor_fp64_lines_body.cuh"
-#include "aderdg_predictor_fp64_prog_body.cuh"
+#include "aderdg_predictor_pencil_body.cuh"
 #include "aderdg_predictor_mixed_prog_body.cuh"
 #include "aderdg_corrector_body.cuh"
 
@@ -65,26 +64,34 @@ struct WorkItem {
 struct EnsArgs {
   SolveDev* solves;
   int nsolves;
+  // the predictor's work items, then the corrector's: the two phases take
+  // blocks of different numbers of cells
   const WorkItem* items;
-  int nitems;
+  int nitems[2];
   int grab;            // work items taken per atomic
   unsigned int* ctr;   // [2] phase counters, reset by phase 3
   int precision;
-  int lines_mask;      // bit N set: order N's predictor uses the line-owner contraction
+  int lines_mask;      // bit N set: order N's predictor uses the pencil (FP64) / line-owner (mixed) form
 };
 
 constexpr int kEnsNT = 128;
 
 constexpr int cmax(int a, int b) { return a > b ? a : b; }
-// default: orders whose predictor runs the line-owner contraction (as the
-// stand-alone kernels do by default: measured faster from order 4 on); the
+// default: the orders whose predictor runs the pencil form in FP64 and the
+// line-owner form in mixed precision instead of node-gather (measured faster
+// for every order in FP64, from order 4 on in mixed precision); the
 // autotuner may choose per order (exa_ensemble_tune_contraction)
-constexpr int kEnsLinesDefault = (1 << 4) | (1 << 5);
+constexpr int kEnsLinesFp64 = (1 << 2) | (1 << 3) | (1 << 4) | (1 << 5);
+constexpr int kEnsLinesMixed = (1 << 4) | (1 << 5);
+// pencil form: cells of an order's block, what kEnsNT threads hold
+constexpr int ens_pencil_cells(int order) { return kEnsNT / ((order + 1) * (order + 1)); }
+template <int N>
+using EnsPencil = PencilShape<2, N, ens_pencil_cells(N)>;
 // shared memory (doubles) the largest 2D order needs in either phase and
-// either contraction
+// either form
 template <int N>
 constexpr int ens_smem_n() {
-  return cmax(cmax(cmax(Fp64LineShape<2, N>::SM_DOUBLES, PredShape<2, N, 0>::SM_DOUBLES),
+  return cmax(cmax(cmax(EnsPencil<N>::SM_DOUBLES, PredShape<2, N, 0>::SM_DOUBLES),
                    cmax(LineShape<2, N>::SM_DOUBLES, MixShape<2, N>::SM_DOUBLES)),
               CorrShapeSmem<2, N>::value);
 }
@@ -143,12 +150,8 @@ __device__ __noinline__ void ens_pred(const SolveDev* sv, int block, double* sme
       if constexpr (N == 5) predictor_mixed_prog_block<2, N, PLANAR>(a, block, smem);
       else predictor_mixed_lines_block<2, N, PLANAR>(a, block, smem);
     }
-    // FP64 order 4: the progressive form (three CTAs per SM in the
-    // per-order launch, 7 % faster); order 5 keeps the line-owner form,
-    // which its registers suit better (measured 10.9 ms per step of a
-    // 512k-cell ensemble against 11.3 ms progressive)
-    else if constexpr (N == 4) predictor_fp64_prog_block<2, N, PLANAR>(a, block, smem);
-    else predictor_fp64_lines_block<2, N, PLANAR>(a, block, smem);
+    // FP64: space-time pencils, cells packed without padding
+    else predictor_pencil_block<2, N, PLANAR, ens_pencil_cells(N)>(a, block, smem);
   } else {
     if (PREC) predictor_mixed_block<2, N, PLANAR>(a, block, smem);
     else predictor_block<2, N, 0, PLANAR, 0>(a, block, smem);
@@ -236,10 +239,11 @@ __device__ __forceinline__ WorkItem ens_segment_item(const EnsArgs& a, int first
   return WorkItem{seg.solve, b - seg.block};
 }
 
-// order 4 in FP64 with the line-owner contraction (the progressive form)
-// is bounded to three CTAs per SM; 0 leaves the others unconstrained
+// the pencil form's registers are bounded for as many CTAs as the
+// stand-alone kernel's (order 5: 200 registers, two CTAs; at three it spills
+// and measured 5 % slower); 0 leaves the others unconstrained
 template <int N, int PREC, bool LINES>
-constexpr int ens_pred_minb() { return (N == 4 && PREC == 0 && LINES) ? 3 : 0; }
+constexpr int ens_pred_minb() { return PREC == 0 && LINES ? (N == 2 ? 5 : (N == 3 ? 4 : (N == 4 ? 3 : 2))) : 0; }
 
 template <int N, int PREC, bool LINES>
 __global__ void __launch_bounds__(kEnsNT, ens_pred_minb<N, PREC, LINES>()) k_ens_pred_order(EnsArgs a, int first, int nseg) {
@@ -269,7 +273,7 @@ __global__ void k_ens_commit(EnsArgs a) {
 template <int N, int PREC, bool LINES>
 constexpr int ens_pred_smem() {
   return LINES ? (PREC ? (N == 5 ? MixProgShape<2, N>::SM_DOUBLES : LineShape<2, N>::SM_DOUBLES)
-                        : (N == 4 ? Fp64ProgShape<2, N>::SM_DOUBLES : Fp64LineShape<2, N>::SM_DOUBLES))
+                        : EnsPencil<N>::SM_DOUBLES)
                : (PREC ? MixShape<2, N>::SM_DOUBLES : PredShape<2, N, 0>::SM_DOUBLES);
 }
 
@@ -279,15 +283,17 @@ __global__ void __launch_bounds__(kEnsNT) k_ensemble_step(EnsArgs a) {
   extern __shared__ double smem[];
   __shared__ int s_item;
   for (int phase = 0; phase < 2; phase++) {
+    const WorkItem* items = a.items + (phase == 0 ? 0 : a.nitems[0]);
+    const int nitems = a.nitems[phase];
     for (;;) {
       if (threadIdx.x == 0) s_item = (int)atomicAdd(&a.ctr[phase], (unsigned)a.grab);
       __syncthreads();
       const int w0 = s_item;
       __syncthreads();
-      if (w0 >= a.nitems) break;
-      const int w1 = min(w0 + a.grab, a.nitems);
+      if (w0 >= nitems) break;
+      const int w1 = min(w0 + a.grab, nitems);
       for (int w = w0; w < w1; w++) {
-        const WorkItem it = a.items[w];
+        const WorkItem it = items[w];
         SolveDev& sv = a.solves[it.solve];
         if (!sv.active) continue;  // uniform across the CTA
         if (phase == 0) run_pred<PREC>(sv, it.block, smem, a.precision, a.lines_mask);
@@ -345,14 +351,14 @@ struct exa_ensemble {
   std::vector<char> used;
   SolveDev* d_solves = nullptr;
   WorkItem* d_items = nullptr;
-  int items_cap = 0, nitems = 0;
+  int items_cap = 0, nitems = 0, ncorr = 0;  // predictor's items, corrector's items after them
   unsigned int* d_ctr = nullptr;
   bool dirty = true;  // solve set changed: rebuild items, re-capture
   bool use_graph = false;
   cudaGraphExec_t graph = nullptr;
   // tuning (exa_ensemble_tune): CTAs per SM, items per grab, order policy
   int ctas_per_sm = 0, grab = 1, order_policy = 0;
-  int lines_mask = kEnsLinesDefault;  // per order: line-owner (bit set) or node-gather contraction
+  int lines_mask = kEnsLinesFp64;  // per order: pencil / line-owner form (bit set) or node-gather
   // launch mode (exa_ensemble_set_launch_mode): 0 one persistent cooperative
   // launch per step; 1 per-order launches (items of an order contiguous)
   int mode = 0;
@@ -362,8 +368,8 @@ struct exa_ensemble {
   cudaStream_t ost[4] = {nullptr, nullptr, nullptr, nullptr};
   cudaEvent_t fork_ev = nullptr;
   cudaEvent_t join_ev[4] = {nullptr, nullptr, nullptr, nullptr};
-  int order_first[6] = {0, 0, 0, 0, 0, 0}, order_count[6] = {0, 0, 0, 0, 0, 0};  // segments per order
-  long order_blocks[6] = {0, 0, 0, 0, 0, 0};  // blocks of cells per order (per-order launches)
+  int order_first[2][6] = {}, order_count[6] = {};  // segments per phase and order
+  long order_blocks[2][6] = {};  // blocks of cells per phase and order (per-order launches)
   bool order_attrs = false;
   int grid = 0;
   std::mutex mu;
@@ -422,7 +428,9 @@ static void arena_free(exa_ensemble* e, size_t off, size_t bytes) {
   }
 }
 
-static int cells_per_block(int order) {
+// cells of a work item of phase 0 (predictor) or 1 (corrector)
+static int cells_per_block(const exa_ensemble* e, int phase, int order) {
+  if (phase == 0 && e->precision != EXA_PREC_MIXED && ((e->lines_mask >> order) & 1)) return ens_pencil_cells(order);
   const int B = order + 1, npc = B * B;
   int g = 1;
   if (npc <= 32) {
@@ -444,11 +452,10 @@ static exa_status_t upload_items(exa_ensemble* e, const std::vector<WorkItem>& i
       return cuda_status(err, "ensemble work items");
     }
   }
-  e->nitems = (int)items.size();
-  if (e->nitems) {
+  if (!items.empty()) {
     // stream-ordered after the launches that read the previous list; a copy
     // from pageable memory is staged before the call returns
-    cudaError_t err = cudaMemcpyAsync(e->d_items, items.data(), sizeof(WorkItem) * e->nitems,
+    cudaError_t err = cudaMemcpyAsync(e->d_items, items.data(), sizeof(WorkItem) * items.size(),
                                       cudaMemcpyHostToDevice, e->st);
     if (err != cudaSuccess) return cuda_status(err, "upload work items");
   }
@@ -457,39 +464,47 @@ static exa_status_t upload_items(exa_ensemble* e, const std::vector<WorkItem>& i
 
 static exa_status_t rebuild_items(exa_ensemble* e) {
   std::vector<WorkItem> items;
-  for (int n = 0; n < 6; n++) e->order_first[n] = e->order_count[n] = e->order_blocks[n] = 0;
-  if (e->mode == 1) {
-    // per-order launches: per order, one segment per active solve holding
-    // the order's running block count at its first block (block field);
-    // CTA b of the order's launch finds its segment by binary search.  Work
-    // on the host is per solve, not per block.
-    std::vector<WorkItem> per[6];
-    for (int s = 0; s < e->max_solves; s++) {
-      if (!e->used[s] || !e->host[s].active) continue;
-      const int n = e->host[s].order;
-      const long nb = (e->host[s].ncells + cells_per_block(n) - 1) / cells_per_block(n);
-      per[n].push_back(WorkItem{s, (int)e->order_blocks[n]});
-      e->order_blocks[n] += nb;
+  auto blocks = [&](int phase, int s) {
+    const int c = cells_per_block(e, phase, e->host[s].order);
+    return (e->host[s].ncells + c - 1) / c;
+  };
+  for (int n = 0; n < 6; n++) e->order_count[n] = 0;
+  for (int phase = 0; phase < 2; phase++) {
+    const size_t first = items.size();
+    for (int n = 0; n < 6; n++) e->order_first[phase][n] = 0, e->order_blocks[phase][n] = 0;
+    if (e->mode == 1) {
+      // per-order launches: per order, one segment per active solve holding
+      // the order's running block count at its first block (block field);
+      // CTA b of the order's launch finds its segment by binary search.  Work
+      // on the host is per solve, not per block.
+      std::vector<WorkItem> per[6];
+      for (int s = 0; s < e->max_solves; s++) {
+        if (!e->used[s] || !e->host[s].active) continue;
+        const int n = e->host[s].order;
+        per[n].push_back(WorkItem{s, (int)e->order_blocks[phase][n]});
+        e->order_blocks[phase][n] += blocks(phase, s);
+      }
+      for (int n = 5; n >= 2; n--) {
+        e->order_first[phase][n] = (int)items.size();
+        e->order_count[n] = (int)per[n].size();
+        items.insert(items.end(), per[n].begin(), per[n].end());
+      }
+    } else {
+      // persistent launch: one work item per block of cells of each active
+      // solve; costly orders first (longest-processing-time order) unless the
+      // policy interleaves
+      for (int s = 0; s < e->max_solves; s++) {
+        if (!e->used[s] || !e->host[s].active) continue;
+        const long nb = blocks(phase, s);
+        for (long b = 0; b < nb; b++) items.push_back(WorkItem{s, (int)b});
+      }
+      if (e->order_policy == 0) {
+        std::stable_sort(items.begin() + first, items.end(), [&](const WorkItem& a, const WorkItem& b) {
+          return e->host[a.solve].order > e->host[b.solve].order;
+        });
+      }
     }
-    for (int n = 5; n >= 2; n--) {
-      e->order_first[n] = (int)items.size();
-      e->order_count[n] = (int)per[n].size();
-      items.insert(items.end(), per[n].begin(), per[n].end());
-    }
-  } else {
-    // persistent launch: one work item per block of cells of each active
-    // solve; costly orders first (longest-processing-time order) unless the
-    // policy interleaves
-    for (int s = 0; s < e->max_solves; s++) {
-      if (!e->used[s] || !e->host[s].active) continue;
-      const long nb = (e->host[s].ncells + cells_per_block(e->host[s].order) - 1) / cells_per_block(e->host[s].order);
-      for (long b = 0; b < nb; b++) items.push_back(WorkItem{s, (int)b});
-    }
-    if (e->order_policy == 0) {
-      std::stable_sort(items.begin(), items.end(), [&](const WorkItem& a, const WorkItem& b) {
-        return e->host[a.solve].order > e->host[b.solve].order;
-      });
-    }
+    (phase == 0 ? e->nitems : e->ncorr) = (int)(items.size() - first);
   }
   if (exa_status_t st = upload_items(e, items)) return st;
   if (e->graph) {
@@ -515,23 +530,23 @@ static cudaError_t set_order_attrs() {
 
 template <int N, int PREC>
 static void launch_pred_order(const EnsArgs& a, const exa_ensemble* e, cudaStream_t st) {
-  const long blocks = e->order_blocks[N];
+  const long blocks = e->order_blocks[0][N];
   if (blocks == 0) return;
   if ((e->lines_mask >> N) & 1)
     k_ens_pred_order<N, PREC, true><<<(unsigned)blocks, kEnsNT, sizeof(double) * ens_pred_smem<N, PREC, true>(), st>>>(
-        a, e->order_first[N], e->order_count[N]);
+        a, e->order_first[0][N], e->order_count[N]);
   else
     k_ens_pred_order<N, PREC, false><<<(unsigned)blocks, kEnsNT, sizeof(double) * ens_pred_smem<N, PREC, false>(),
-                                       st>>>(a, e->order_first[N], e->order_count[N]);
+                                       st>>>(a, e->order_first[0][N], e->order_count[N]);
   count_launch();
 }
 
 template <int N>
 static void launch_corr_order(const EnsArgs& a, const exa_ensemble* e, cudaStream_t st) {
-  const long blocks = e->order_blocks[N];
+  const long blocks = e->order_blocks[1][N];
   if (blocks == 0) return;
   k_ens_corr_order<N><<<(unsigned)blocks, kEnsNT, sizeof(double) * CorrShapeSmem<2, N>::value, st>>>(
-      a, e->order_first[N], e->order_count[N]);
+      a, e->order_first[1][N], e->order_count[N]);
   count_launch();
 }
 
@@ -549,7 +564,7 @@ static exa_status_t launch_step_orders(exa_ensemble* e, const EnsArgs& a) {
   // nothing until the commit), costly orders issued first
   cudaError_t err = cudaEventRecord(e->fork_ev, e->st);
   for (int n = 5; n >= 2 && err == cudaSuccess; n--) {
-    if (e->order_blocks[n] == 0) continue;
+    if (e->order_blocks[0][n] == 0) continue;
     cudaStream_t os = e->ost[n - 2];
     err = cudaStreamWaitEvent(os, e->fork_ev, 0);
     if (err != cudaSuccess) break;
@@ -573,7 +588,8 @@ static exa_status_t launch_step(exa_ensemble* e) {
   a.solves = e->d_solves;
   a.nsolves = e->max_solves;
   a.items = e->d_items;
-  a.nitems = e->nitems;
+  a.nitems[0] = e->nitems;
+  a.nitems[1] = e->ncorr;
   a.grab = e->grab;
   a.ctr = e->d_ctr;
   a.precision = e->precision;
@@ -654,6 +670,7 @@ exa_status_t exa_ensemble_create(int precision, int max_solves, size_t arena_byt
   exa_ensemble* e = new (std::nothrow) exa_ensemble;
   if (!e) return set_error(EXA_ENOMEM, "host allocation");
   e->precision = precision;
+  e->lines_mask = precision == EXA_PREC_MIXED ? kEnsLinesMixed : kEnsLinesFp64;
   e->max_solves = max_solves;
   e->arena_bytes = arena_bytes;
   cudaGetDevice(&e->device);
