@@ -213,6 +213,18 @@ __device__ __forceinline__ void corrector_block(const CorrArgs& a, long block, d
     }
     __syncthreads();
   }
+  // each face value's Rusanov flux once, over the own flux
+  // (riemannSolverNonlinear.cpph:83-115: F = (FL+FR)/2 - smax/2 (QR-QL), left
+  // = lower cell; face 2d+1: this cell is the left one, face 2d: the right
+  // one).  The B nodes that apply a face value then read one double instead
+  // of forming it from four.
+  if (valid)
+    for (int k = s; k < FV; k += G) {
+      const int f = k / (NF * V);
+      const double dq = sQn[k] - sQo[k];
+      sFo[k] = 0.5 * (sFn[k] + sFo[k]) - 0.5 * sSm[f] * ((f & 1) ? dq : -dq);
+    }
+  __syncthreads();
   double dtc = DBL_MAX;
   if (valid && s < NPC) {
     int sd[3];
@@ -224,9 +236,7 @@ __device__ __forceinline__ void corrector_block(const CorrArgs& a, long block, d
 #pragma unroll
     for (int m = 0; m < V; m++) v[m] = v_lduh[m];
     // surface integral (surfaceIntegralNonlinear.cpph:21-85) of the Rusanov
-    // fluxes at this node's face nodes (riemannSolverNonlinear.cpph:83-115:
-    // F = (FL+FR)/2 - smax/2 (QR-QL), left = lower cell), formed here by
-    // each node that applies them instead of being stored first
+    // fluxes at this node's face nodes
 #pragma unroll
     for (int d = 0; d < DIM; d++) {
       double wprod = 1.0;
@@ -237,14 +247,8 @@ __device__ __forceinline__ void corrector_block(const CorrArgs& a, long block, d
       const int j = face_node<DIM, B>(sd, d);
       const double cr = T.fr[sd[d]], cl = T.fl[sd[d]];
       const int kr = ((2 * d + 1) * NF + j) * V, kl = ((2 * d) * NF + j) * V;
-      const double smr = sSm[2 * d + 1], sml = sSm[2 * d];
 #pragma unroll
-      for (int m = 0; m < V; m++) {
-        // face 2d+1: this cell is the left one; face 2d: the right one
-        const double FR_ = 0.5 * (sFn[kr + m] + sFo[kr + m]) - 0.5 * smr * (sQn[kr + m] - sQo[kr + m]);
-        const double FL_ = 0.5 * (sFo[kl + m] + sFn[kl + m]) - 0.5 * sml * (sQo[kl + m] - sQn[kl + m]);
-        v[m] -= (FR_ * cr - FL_ * cl) * us;
-      }
+      for (int m = 0; m < V; m++) v[m] -= (sFo[kr + m] * cr - sFo[kl + m] * cl) * us;
     }
     // solution update (solutionUpdate.cpph:23-47)
     double W = 1.0;
