@@ -158,14 +158,10 @@ __device__ __forceinline__ void predictor_pencil_block(const PredArgs& a, long b
 
   // ---- first iteration: the iterate is luh in every slice, so one slice is
   // evaluated and every other takes its values
-  bool lost = true;  // every value of this thread's node is NaN
   if (valid) {
     double u[V], F[DIM][V];
 #pragma unroll
-    for (int m = 0; m < V; m++) {
-      u[m] = luh[s * V + m];
-      lost = lost && isnan(u[m]);
-    }
+    for (int m = 0; m < V; m++) u[m] = luh[s * V + m];
     euler_flux<DIM, PLANAR>(u, F);
 #pragma unroll
     for (int m = 0; m < V; m++) {
@@ -174,10 +170,8 @@ __device__ __forceinline__ void predictor_pencil_block(const PredArgs& a, long b
       if (DIM == 3) sF2[node + m] = F[DIM - 1][m];
     }
   }
-  // Cells with nothing but NaN (a run that has blown up) would iterate to the
-  // limit, 2(N+1) times, and give NaN everywhere: the outcome is known.
-  lost = __syncthreads_and(lost);
-  if (valid && !lost)
+  __syncthreads();
+  if (valid)
 #pragma unroll
     for (int r = 0; r < S::T_ROUNDS; r++) {
       const int k = s + r * TPC;
@@ -254,11 +248,19 @@ __device__ __forceinline__ void predictor_pencil_block(const PredArgs& a, long b
     for (int m = 0; m < V; m++) q[x][m] = valid ? luh[sl * R5 + x * V + m] : 0.0;
   __syncthreads();
 
-  int it = lost ? MAXIT : 0;
+  int it = 0;
   // done: this thread's cell has its outputs' values (uniform over the CTA
   // with one cell; threads without a cell are done after one iteration)
   bool conv = false, done = false;
-  for (int iter = 0; !lost; iter++) {
+  // lost: the last residual was NaN.  A cell of nothing but NaN (a run that has
+  // blown up) would iterate to the limit, 2(N+1) times, and stay NaN, each value
+  // being a sum over the others.  A thread whose pencil holds only NaN would
+  // make the residual NaN again; it adds kVote in its stead, and a sum of TPC
+  // votes (exact, and out of reach for fewer: the others add no less than 0) ends
+  // the cell.  Any other sum with a vote in it is not below the tolerance.
+  constexpr double kVote = -0x1p1000;
+  bool lost = false;
+  for (int iter = 0;; iter++) {
     // the new pencil and its squared increment
     double qn[B][V], r2 = 0.0;
     if (valid && !done)
@@ -271,10 +273,19 @@ __device__ __forceinline__ void predictor_pencil_block(const PredArgs& a, long b
           r2 += d * d;
           if (kHold) qn[x][m] = v;
         }
+    if (lost && valid && !done) {
+      bool all = true;
+#pragma unroll
+      for (int x = 0; x < B; x++)
+#pragma unroll
+        for (int m = 0; m < V; m++) all = all && isnan(q[x][m]);
+      if (all) r2 = kVote;
+    }
     const double res = pencil_sum<S>(r2, lc, s, sred, iter);
     if (!done) {
-      it = iter + 1;
-      conv = res < 1e-7 * 1e-7;
+      it = res == TPC * kVote ? MAXIT : iter + 1;
+      conv = res >= 0.0 && res < 1e-7 * 1e-7;
+      lost = !(res >= 0.0);
       done = conv || it == MAXIT;
       // the outputs need the last iteration's input (for its flux), put in
       // F_y's place, and its result, over G
@@ -404,15 +415,7 @@ __device__ __forceinline__ void predictor_pencil_block(const PredArgs& a, long b
 #pragma unroll
     for (int d = 0; d < DIM; d++) fa[d][m] = 0.0;
   }
-  if (valid && lost) {
-    // (one NaN of luh stands for all)
-#pragma unroll
-    for (int m = 0; m < V; m++) {
-      qh[m] = luh[s * V + m];
-#pragma unroll
-      for (int d = 0; d < DIM; d++) fa[d][m] = qh[m];
-    }
-  } else if (valid)
+  if (valid)
 #pragma unroll
     for (int n = 0; n < B; n++) {
       double u[V], F[DIM][V];

@@ -61,3 +61,29 @@ def test_pencil_vs_gather_and_oracle(dim, order, cells, planar):
                 min(dx) if n == 'lduh' else 1.0)
             assert np.abs(a[n][c] - ref).max() <= tol, (n, c)
             assert np.abs(a[n][c] - b[n][c]).max() <= tol, (n, c)
+
+
+@pytest.mark.parametrize('dim,order,cells', [(2, 2, 29), (2, 3, 17), (2, 4, 11), (2, 5, 8), (3, 3, 5), (3, 4, 4),
+                                             (3, 5, 3)])
+def test_cells_of_nan(dim, order, cells):
+    """Cells of nothing but NaN, cells with one NaN, and the cells beside them:
+    the iteration limit and NaN for the first two, what they are alone for the
+    others."""
+    rng = np.random.default_rng(dim + order)
+    nn = (order + 1) ** dim
+    q = np.zeros((cells, nn, V))
+    q[..., 0] = 1.0 + 0.1 * rng.random((cells, nn))
+    q[..., 1:4] = 0.1 * rng.standard_normal((cells, nn, 3))
+    q[..., 4] = 2.5 + 0.1 * rng.random((cells, nn))
+    dx, dt = [0.05, 0.04, 0.03][:dim], 3e-4
+    good, ig = run(0, dim, order, cells, q, dx, dt, E.PDE_EULER)
+    q[0] = np.nan
+    q[2, nn // 2, 1] = np.nan
+    a, ia = run(0, dim, order, cells, q, dx, dt, E.PDE_EULER)
+    for c in range(cells):
+        if c in (0, 2):
+            assert ia[c] == 2 * (order + 1)
+            assert all(np.isnan(a[n][c]).all() for n in a)
+        else:
+            assert ia[c] == ig[c]
+            assert all(np.array_equal(a[n][c], good[n][c]) for n in a)
