@@ -62,9 +62,12 @@ __device__ __forceinline__ void corrector_block(const CorrArgs& a, long block, d
 
   int cc[3] = {0, 0, 0};
   if (valid) {
-    cc[0] = (int)(cell % a.n[0]);
-    cc[1] = (int)((cell / a.n[0]) % a.n[1]);
-    cc[2] = DIM == 3 ? (int)(cell / ((long)a.n[0] * a.n[1])) : 0;
+    // 32-bit divisions: the 64-bit ones were a fifth of the kernel's
+    // instructions (a grid's cells are far below 2^31: each holds > 1 KB)
+    const unsigned c = (unsigned)cell, row = c / (unsigned)a.n[0];
+    cc[0] = (int)(c - row * (unsigned)a.n[0]);
+    cc[2] = DIM == 3 ? (int)(row / (unsigned)a.n[1]) : 0;
+    cc[1] = (int)row - cc[2] * a.n[1];
   }
   // Own faces and the matching faces of the neighbours -> shared memory,
   // as asynchronous 8-byte copies (cp.async): every copy of the CTA is in
@@ -225,7 +228,7 @@ __device__ __forceinline__ void corrector_block(const CorrArgs& a, long block, d
       sFo[k] = 0.5 * (sFn[k] + sFo[k]) - 0.5 * sSm[f] * ((f & 1) ? dq : -dq);
     }
   __syncthreads();
-  double dtc = DBL_MAX;
+  double den = 0.0;  // sum over directions of |lambda|_max / dx
   if (valid && s < NPC) {
     int sd[3];
     sd[0] = s % B;
@@ -243,7 +246,7 @@ __device__ __forceinline__ void corrector_block(const CorrArgs& a, long block, d
 #pragma unroll
       for (int e = DIM - 1; e >= 0; e--)
         if (e != d) wprod *= T.w[sd[e]];
-      const double us = wprod / a.dx[d];
+      const double us = wprod * a.idx[d];
       const int j = face_node<DIM, B>(sd, d);
       const double cr = T.fr[sd[d]], cl = T.fl[sd[d]];
       const int kr = ((2 * d + 1) * NF + j) * V, kl = ((2 * d) * NF + j) * V;
@@ -254,8 +257,7 @@ __device__ __forceinline__ void corrector_block(const CorrArgs& a, long block, d
     double W = 1.0;
 #pragma unroll
     for (int e = DIM - 1; e >= 0; e--) W *= T.w[sd[e]];
-    const double dt = *a.dt_dev;
-    const double us = dt / W;
+    const double us = *a.dt_dev / W;
     double q[V];
     bool finite = true;
 #pragma unroll
@@ -267,22 +269,23 @@ __device__ __forceinline__ void corrector_block(const CorrArgs& a, long block, d
     if (!finite && a.nan_flag) atomicOr(a.nan_flag, 1);
     // next step's stable dt at this node (stableTimeStepSize.cpph:21-61)
     if (a.dt_next) {
-      double den = 0.0;
 #pragma unroll
-      for (int d = 0; d < DIM; d++) den += euler_max_eig<PLANAR>(q, d) / a.dx[d];
-      dtc = a.dt_factor / den;
+      for (int d = 0; d < DIM; d++) den += euler_max_eig<PLANAR>(q, d) * a.idx[d];
     }
   }
   if (a.dt_next) {
-    // minimum over the warp's lanes of this cell, then one atomic per warp
-    // (per cell for cells narrower than a warp), skipped when the slot
-    // already holds a smaller value (read at L2, where the atomics land;
-    // the slot only decreases within a step)
-    constexpr int L = G < 32 ? G : 32;
+    // largest sum over the warp's lanes (of all its cells: one grid, one dt;
+    // the division is monotone, so dt_factor / largest is the smallest dt),
+    // then one atomic per warp, skipped when the slot already holds a smaller
+    // value (read at L2, where the atomics land; the slot only decreases
+    // within a step)
 #pragma unroll
-    for (int o = L / 2; o > 0; o >>= 1) dtc = fmin(dtc, __shfl_xor_sync(0xffffffffu, dtc, o));
-    if (valid && (s % L) == 0 && dtc < __longlong_as_double((long long)__ldcg(a.dt_next)))
-      atomic_min_pos_double(a.dt_next, dtc);
+    for (int o = 16; o > 0; o >>= 1) den = fmax(den, __shfl_xor_sync(0xffffffffu, den, o));
+    if ((threadIdx.x & 31) == 0) {
+      // (cells padded with idle lanes bound the slot even when all is NaN)
+      const double dtn = a.dt_factor / den, dtc = NPC < G ? fmin(DBL_MAX, dtn) : dtn;
+      if (dtc < __longlong_as_double((long long)__ldcg(a.dt_next))) atomic_min_pos_double(a.dt_next, dtc);
+    }
   }
 }
 

@@ -24,6 +24,13 @@ __global__ void __launch_bounds__(CellShape<DIM, N>::NT) k_corrector(CorrArgs a)
   corrector_block<DIM, N, PLANAR>(a, blockIdx.x, smem);
 }
 
+// Shared-memory carveout, in percent: the faces' values, lduh, luh and the
+// staged tables also pass through L1, which the default carveout leaves too
+// little of.  50^3 cells of order 4: 1140..1160 us at the default, 86 and 100,
+// 978 at 72, 1026 at 58, 1313 at 43 (fewer CTAs); the other orders and 2D are
+// best or level at 72 too.
+constexpr int kCorrectorCarveout = 72;
+
 exa_status_t launch_corrector(int dim, int order, int pde, const CorrArgs& a, cudaStream_t st) {
   const bool planar = pde == EXA_PDE_EULER_PLANAR;
 #define EXA_CORR(D_, N_, P_)                                                                 \
@@ -32,6 +39,8 @@ exa_status_t launch_corrector(int dim, int order, int pde, const CorrArgs& a, cu
     auto kern = k_corrector<D_, N_, P_>;                                                     \
     const size_t sm = sizeof(double) * CorrShapeSmem<D_, N_>::value;                         \
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); \
+    if (e == cudaSuccess)                                                                    \
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, kCorrectorCarveout); \
     if (e != cudaSuccess) return cuda_status(e, "corrector attribute");                      \
     const long nb = (a.ncells + S::CPB - 1) / S::CPB;                                        \
     if (nb <= 0) return EXA_OK;                                                              \

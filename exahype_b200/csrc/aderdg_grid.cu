@@ -223,7 +223,7 @@ static exa_status_t grid_correct(exa_aderdg_grid* g) {
   c.ncells = g->ncells;
   for (int i = 0; i < 3; i++) {
     c.n[i] = i < g->cfg.dim ? g->cfg.n[i] : 1;
-    c.dx[i] = g->desc.dx[i];
+    c.idx[i] = 1.0 / g->desc.dx[i];
   }
   c.dt_dev = &g->gd->dt;
   c.luh = g->luh;

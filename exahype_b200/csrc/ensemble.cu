@@ -38,7 +38,7 @@ double host_pnpm(int order);
 struct SolveDev {
   int order, pde, dt_policy, active;  // active: 1 while steps remain
   int n[2];
-  double dx[2];
+  double dx[2], idx[2];  // cell sizes and their reciprocals
   long ncells;
   double* luh;
   double* lduh;
@@ -103,8 +103,8 @@ __device__ __forceinline__ PredArgs pred_args(const SolveDev& sv, int precision)
   a.luh = sv.luh;
   a.dt = 0.0;
   a.dt_dev = &sv.dt;
-  a.idx[0] = 1.0 / sv.dx[0];
-  a.idx[1] = 1.0 / sv.dx[1];
+  a.idx[0] = sv.idx[0];
+  a.idx[1] = sv.idx[1];
   a.idx[2] = 0.0;
   a.lduh = sv.lduh;
   a.lQhbnd = sv.qb;
@@ -121,9 +121,9 @@ __device__ __forceinline__ CorrArgs corr_args(SolveDev& sv) {
   c.n[0] = sv.n[0];
   c.n[1] = sv.n[1];
   c.n[2] = 1;
-  c.dx[0] = sv.dx[0];
-  c.dx[1] = sv.dx[1];
-  c.dx[2] = 1.0;
+  c.idx[0] = sv.idx[0];
+  c.idx[1] = sv.idx[1];
+  c.idx[2] = 1.0;
   c.dt_dev = &sv.dt;
   c.luh = sv.luh;
   c.lduh = sv.lduh;
@@ -744,6 +744,7 @@ exa_status_t exa_ensemble_add(exa_ensemble* e, const exa_solve_config_t* c, long
   sv.n[1] = c->n[1];
   sv.dx[0] = c->length[0] / c->n[0];
   sv.dx[1] = c->length[1] / c->n[1];
+  for (int d = 0; d < 2; d++) sv.idx[d] = 1.0 / sv.dx[d];
   sv.ncells = nc;
   char* base = e->arena + off;
   sv.luh = (double*)base;
@@ -936,6 +937,7 @@ exa_status_t exa_ensemble_restore(exa_ensemble* e, const exa_solve_config_t* c, 
   sv.n[1] = c->n[1];
   sv.dx[0] = c->length[0] / c->n[0];
   sv.dx[1] = c->length[1] / c->n[1];
+  for (int d = 0; d < 2; d++) sv.idx[d] = 1.0 / sv.dx[d];
   sv.ncells = nc;
   char* base = e->arena + off;
   sv.luh = (double*)base;

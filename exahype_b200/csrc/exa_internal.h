@@ -64,7 +64,7 @@ exa_status_t launch_predictor_mixed(const exa_aderdg_desc_t& d, const PredArgs& 
 struct CorrArgs {
   long ncells;
   int n[3];
-  double dx[3];
+  double idx[3];            // 1/dx
   const double* dt_dev;     // dt of this step
   double* luh;
   const double* lduh;
