@@ -12,13 +12,12 @@
 //
 // The reference evaluates every projection as a direct B^dim-term sum per
 // output point.  The operators are tensor products of one 1D table, so here
-// they are applied as dim one-dimensional passes (sum factorisation) in
-// shared memory: a pass reads each line of its input once into registers
-// and writes all outputs of the line, with the table entries as
-// compile-time constant-bank operands (order is a template parameter).
-// Several cells share a CTA so that every pass has enough lines for the
-// 256 threads; threads take (cell, line, variable) items with the variable
-// fastest, so the final pass's global stores are contiguous runs.
+// they are applied as dim one-dimensional sums, and a thread keeps all of them
+// for one output column (x, variable) in registers: its x sums from the cell's
+// staged values (loads that the lanes of one variable share, one wavefront
+// each), then y, then z.  No intermediate arrays and no pass over them;
+// consecutive lanes hold consecutive (x, variable), so stores run over whole
+// rows.
 //
 // Layouts (the reference's, KernelUtils.h idx4): luh [z][y][x][nvar] with B
 // points per direction; lim [z][y][x][nvar] with S + 2g points per
@@ -38,6 +37,8 @@ namespace exa {
 
 constexpr int kLimMaxOrder = 6;  // B <= 7, S <= 13
 constexpr int kLimNT = 256;
+constexpr int kLimColNT = 128;  // threads of the projections
+constexpr int kLimMmNT = 128;   // and of the extrema
 constexpr int kLimMaxSmem = 200 * 1024;
 
 struct LimConst {
@@ -60,139 +61,19 @@ __device__ __forceinline__ double lim_coef(int p, int m) {
 __device__ __forceinline__ double lim_min(double a, double b) { return b < a ? b : a; }
 __device__ __forceinline__ double lim_max(double a, double b) { return a < b ? b : a; }
 
-// One 1D pass: applies table TAB (NI inputs -> NO outputs, T[p][m]) along
-// direction D of a point array of extents EX x EY x EZ (x fastest), for
-// `ncell` cells and variables v < nv.  Input point p of cell c starts at
-// in + c * cs_in + p * ps_in.  Each thread takes (cell, line, variable)
-// items, the variable fastest, starting with item (threadIdx.x - t0) mod NT
-// (t0 lets a pass continue where the previous pass of the same phase left
-// the threads); it hands the inputs and the NO outputs of its line to
-// out.line<D>(c, x, y, z, v, inputs, outputs, item) with the D coordinate
-// of (x, y, z) 0.  Strides and counts are plain ints: with the variable
-// count a compile-time constant in the caller they fold into immediate
-// offsets.
-template <int TAB, int B, int EX, int EY, int EZ, int D, int NO, class Out>
-__device__ __forceinline__ void lim_pass(const double* in, int ps_in, int cs_in, int ncell, int nv, Out& out,
-                                         int t0 = 0) {
-  constexpr int NI = D == 0 ? EX : (D == 1 ? EY : EZ);
-  constexpr int LINES = EX * EY * EZ / NI;
-  constexpr int SD = D == 0 ? 1 : (D == 1 ? EX : EX * EY);
-  const int items = ncell * LINES * nv;
-  for (int it = (threadIdx.x + kLimNT - t0 % kLimNT) % kLimNT; it < items; it += kLimNT) {
-    const int v = it % nv;
-    const int line = (it / nv) % LINES;
-    const int c = it / (nv * LINES);
-    int x = 0, y = 0, z = 0;
-    if (D == 0) {
-      y = line % EY;
-      z = line / EY;
-    } else if (D == 1) {
-      x = line % EX;
-      z = line / EX;
-    } else {
-      x = line % EX;
-      y = line / EX;
-    }
-    const double* src = in + c * cs_in + ((z * EY + y) * EX + x) * ps_in + v;
-    double a[NI];
-#pragma unroll
-    for (int p = 0; p < NI; p++) a[p] = src[p * SD * ps_in];
-    double o[NO];
-#pragma unroll
-    for (int m = 0; m < NO; m++) {
-      double acc = 0.0;
-#pragma unroll
-      for (int p = 0; p < NI; p++) acc = fma(lim_coef<TAB, B>(p, m), a[p], acc);
-      o[m] = acc;
-    }
-    out.template line<D, NI, NO>(c, x, y, z, v, a, o, it);
-  }
-}
-
-// writes a pass's outputs to a shared-memory array of extents ox x oy x .
-struct SmemOut {
-  double* base;
-  int ps, cs, ox, oy;
-  template <int D, int NI, int NO>
-  __device__ __forceinline__ void line(int c, int x, int y, int z, int v, const double (&)[NI],
-                                       const double (&o)[NO], int) {
-    double* p = base + c * cs + ((z * oy + y) * ox + x) * ps + v;
-    const int st = D == 0 ? ps : (D == 1 ? ox * ps : ox * oy * ps);
-#pragma unroll
-    for (int m = 0; m < NO; m++) p[m * st] = o[m];
-  }
+// CTAs per SM that the projections' registers are bounded for: the most that
+// compile (nearly) without spills.  In DG -> FV a reload waits behind the row's
+// stores: 40 bytes of them cost a third of the kernel.
+template <int DIM, int B, bool TO_FV>
+struct LimMinB {
+  static constexpr int fv[8] = {0, 0, 8, 8, 5, 4, 2, 2}, dg[8] = {0, 0, 8, 8, 6, 5, 3, 2};  // by B
+  static constexpr int value = DIM == 2 ? 8 : (TO_FV ? fv[B] : dg[B]);
 };
-
-// writes to the interior of ghosted global patches (or plain luh arrays:
-// off = 0, ext = B)
-template <int DIM>
-struct GlobalOut {
-  double* base;  // cell 0 of the array
-  long cs;       // doubles per cell
-  int nvar, ext, off;
-  long c0;       // first cell (selection index) of the CTA
-  const int* list;
-  template <int D, int NI, int NO>
-  __device__ __forceinline__ void line(int c, int x, int y, int z, int v, const double (&)[NI],
-                                       const double (&o)[NO], int) {
-    const long pt = DIM == 3 ? ((long)(z + off) * ext + (y + off)) * ext + (x + off) : (long)(y + off) * ext + (x + off);
-    const long cell = list ? (long)list[c0 + c] : c0 + c;
-    double* p = base + cell * cs + pt * nvar + v;
-    const long st = (D == 0 ? 1L : (D == 1 ? (long)ext : (long)ext * ext)) * nvar;
-#pragma unroll
-    for (int m = 0; m < NO; m++) p[m * st] = o[m];
-  }
-};
-
-// extrema of the outputs of a line, stored per item
-struct MinMaxOut {
-  double* pmn;
-  double* pmx;
-  template <int D, int NI, int NO>
-  __device__ __forceinline__ void line(int, int, int, int, int, const double (&)[NI], const double (&o)[NO],
-                                       int it) {
-    double mn = o[0], mx = o[0];
-#pragma unroll
-    for (int m = 1; m < NO; m++) {
-      mn = lim_min(mn, o[m]);
-      mx = lim_max(mx, o[m]);
-    }
-    pmn[it] = mn;
-    pmx[it] = mx;
-  }
-};
-
-// a shared-memory store plus the extrema of the pass's INPUT line (the
-// nodes themselves, seen by the first pass over luh)
-struct SmemOutInputMinMax {
-  SmemOut s;
-  double* pmn;
-  double* pmx;
-  template <int D, int NI, int NO>
-  __device__ __forceinline__ void line(int c, int x, int y, int z, int v, const double (&a)[NI],
-                                       const double (&o)[NO], int it) {
-    s.line<D, NI, NO>(c, x, y, z, v, a, o, it);
-    double mn = a[0], mx = a[0];
-#pragma unroll
-    for (int p = 1; p < NI; p++) {
-      mn = lim_min(mn, a[p]);
-      mx = lim_max(mx, a[p]);
-    }
-    pmn[it] = mn;
-    pmx[it] = mx;
-  }
-};
-
-// cooperative copy of `n` doubles (global -> shared)
-__device__ __forceinline__ void lim_copy_in(double* dst, const double* src, long n) {
-  for (long i = threadIdx.x; i < n; i += kLimNT) dst[i] = src[i];
-}
-
-template <int B>
-struct LimOcc {
-  // resident CTAs per SM the kernels are compiled for (register budget of
-  // 64 / 85 / 255 per thread: the least that compiles without spills)
-  static constexpr int value = B <= 4 ? 4 : (B == 5 ? 3 : 1);
+// and those of the extrema
+template <int DIM, int B, bool WALK>
+struct LimMmMinB {
+  static constexpr int walk[8] = {0, 0, 8, 8, 7, 3, 3, 3}, col[8] = {0, 0, 8, 8, 6, 5, 3, 2};
+  static constexpr int value = WALK ? walk[B] : (DIM == 2 ? 8 : col[B]);
 };
 
 // Optional cell selection: the kernels run on cells list[0 .. *count) (at
@@ -207,61 +88,91 @@ struct LimSel {
   __device__ __forceinline__ long cell(long k) const { return list ? (long)list[k] : k; }
 };
 
-// copies the selected cells' input arrays (n doubles each) to shared memory
-__device__ __forceinline__ void lim_copy_cells(double* dst, const double* src, int n, long c0, int nc,
-                                               const LimSel& sel) {
+// starts copying the selected cells' luh (n doubles each) to shared memory,
+// every copy in flight at once (a load-store loop waited for each few); the
+// caller waits (cp_async_commit_wait_all) and has a barrier
+__device__ __forceinline__ void lim_stage_cells(double* dst, const double* __restrict__ src, int n, long c0, int nc,
+                                                const LimSel& sel, int nt) {
   if (!sel.list) {
-    lim_copy_in(dst, src + c0 * n, (long)nc * n);
-    return;
-  }
-  for (int i = threadIdx.x; i < nc * n; i += kLimNT) {
-    const int c = i / n;
-    dst[i] = src[sel.cell(c0 + c) * n + (i - c * n)];
+    for (int i = threadIdx.x; i < nc * n; i += nt) cp_async8(dst + i, src + c0 * n + i);
+  } else {
+    for (int i = threadIdx.x; i < nc * n; i += nt) {
+      const int c = i / n;
+      cp_async8(dst + i, src + sel.cell(c0 + c) * n + (i - c * n));
+    }
   }
 }
 
 // ------------------------------------------------------------ DG -> FV
-// shared memory per cell (doubles per variable): luh, pass-x and pass-y
-// results (3D)
-template <int DIM, int B>
-__host__ __device__ constexpr int lim_to_fv_cell_doubles_per_var() {
-  return DIM == 3 ? B * B * B + B * B * (2 * B - 1) + B * (2 * B - 1) * (2 * B - 1) : B * B + B * (2 * B - 1);
-}
-
-// NVT: the variable count when known at compile time (0 = runtime nvar)
+// One thread per (cell, subcell column x, variable): the x sums of its
+// column for every (z, y) in registers (B^2 doubles), then for every row of
+// subcells the y sums and the z sums, stored as they are formed.  A CTA
+// stages and serves cpb cells.  Bound by the stores (rows of S * nvar doubles
+// that start and end inside a sector): ghosted patches (2 layers) leave at 2.3
+// to 3 TB/s.  Per call, the passes through shared memory of before -> now:
+// 24,000 3D cells of order 4 326 -> 313 us, 13,888 of order 5 555 -> 296, 8,746
+// of order 6 551 -> 322, 166,666 2D cells of order 5 675 -> 334, 240,000 of
+// order 4 405 -> 342; 3D orders 1 to 3 level (317 -> 320 at order 3).
 template <int DIM, int B, int NVT>
-__global__ void __launch_bounds__(kLimNT, LimOcc<B>::value)
-    k_lim_to_fv(int nvar_rt, int ghost, long ncells, int cpb, const double* luh, double* lim, LimSel sel) {
-  constexpr int S = 2 * B - 1;
-  constexpr int NPC = DIM == 3 ? B * B * B : B * B;
+__global__ void __launch_bounds__(kLimColNT, LimMinB<DIM, B, true>::value)
+    k_lim_to_fv(int nvar_rt, int ghost, long ncells, int cpb, const double* __restrict__ luh, double* lim,
+                LimSel sel) {
+  constexpr int S = 2 * B - 1, BZ = DIM == 3 ? B : 1, SZ = DIM == 3 ? S : 1, NPC = BZ * B * B;
   const int nvar = NVT ? NVT : nvar_rt;
+  const int SG = S + 2 * ghost;
+  const long row = (long)SG * nvar, plane = row * SG;
   extern __shared__ double sm[];
+  __shared__ double sT[S * B];  // means table, [subcell][node]
+  for (int i = threadIdx.x; i < S * B; i += blockDim.x) sT[i] = c_lim[B - 1].uh2lim[i % B][i / B];
   const long nce = sel.cells(ncells);
-  // one cell block per iteration (a single one unless a selection launched
-  // fewer CTAs than blocks)
   for (long c0 = (long)blockIdx.x * cpb; c0 < nce; c0 += (long)gridDim.x * cpb) {
     const int nc = (int)min((long)cpb, nce - c0);
-    const int SG = S + 2 * ghost;
-    const long lim_cell = (long)nvar * (DIM == 3 ? SG * SG * SG : SG * SG);
-    double* A = sm;
-    double* T1 = A + cpb * NPC * nvar;
-    lim_copy_cells(A, luh, NPC * nvar, c0, nc, sel);
+    lim_stage_cells(sm, luh, NPC * nvar, c0, nc, sel, blockDim.x);
+    cp_async_commit_wait_all();
     __syncthreads();
-    GlobalOut<DIM> go{lim, lim_cell, nvar, SG, ghost, c0, sel.list};
-    if (DIM == 2) {
-      SmemOut o1{T1, nvar, S * B * nvar, S, B};
-      lim_pass<kTabUh2Lim, B, B, B, 1, 0, S>(A, nvar, NPC * nvar, nc, nvar, o1);
-      __syncthreads();
-      lim_pass<kTabUh2Lim, B, S, B, 1, 1, S>(T1, nvar, S * B * nvar, nc, nvar, go);
-    } else {
-      double* T2 = T1 + cpb * B * B * S * nvar;
-      SmemOut o1{T1, nvar, B * B * S * nvar, S, B};
-      lim_pass<kTabUh2Lim, B, B, B, B, 0, S>(A, nvar, NPC * nvar, nc, nvar, o1);
-      __syncthreads();
-      SmemOut o2{T2, nvar, B * S * S * nvar, S, S};
-      lim_pass<kTabUh2Lim, B, S, B, B, 1, S>(T1, nvar, B * B * S * nvar, nc, nvar, o2);
-      __syncthreads();
-      lim_pass<kTabUh2Lim, B, S, S, B, 2, S>(T2, nvar, B * S * S * nvar, nc, nvar, go);
+    for (int it = threadIdx.x; it < nc * S * nvar; it += blockDim.x) {
+      const int v = it % nvar, x = (it / nvar) % S, c = it / (nvar * S);
+      const double* src = sm + c * NPC * nvar + v;
+      double cx[B];
+#pragma unroll
+      for (int p = 0; p < B; p++) cx[p] = sT[x * B + p];
+      double a[BZ][B];
+#pragma unroll
+      for (int z = 0; z < BZ; z++)
+#pragma unroll
+        for (int y = 0; y < B; y++) {
+          double acc = 0.0;
+#pragma unroll
+          for (int p = 0; p < B; p++) acc = fma(cx[p], src[((z * B + y) * B + p) * nvar], acc);
+          a[z][y] = acc;
+        }
+      double* dst = lim + sel.cell(c0 + c) * (DIM == 3 ? plane * SG : plane) + (DIM == 3 ? ghost * plane : 0) +
+                    ghost * row + (long)(ghost + x) * nvar + v;
+      // (a loop, its coefficients in shared memory: unrolled, the y sums of
+      // several rows live at once and spill)
+#pragma unroll 1
+      for (int y = 0; y < S; y++) {
+        double b[BZ];
+#pragma unroll
+        for (int z = 0; z < BZ; z++) {
+          double acc = 0.0;
+#pragma unroll
+          for (int p = 0; p < B; p++) acc = fma(sT[y * B + p], a[z][p], acc);
+          b[z] = acc;
+        }
+        double* d = dst + y * row;
+        if (DIM == 2) {
+          d[0] = b[0];
+        } else {
+#pragma unroll
+          for (int z = 0; z < SZ; z++) {
+            double acc = 0.0;
+#pragma unroll
+            for (int p = 0; p < BZ; p++) acc = fma(c_lim[B - 1].uh2lim[p][z], b[p], acc);
+            d[z * plane] = acc;
+          }
+        }
+      }
     }
     __syncthreads();
   }
@@ -300,137 +211,334 @@ __device__ __forceinline__ void lim_stage_interior(double* A, const double* __re
 }
 
 // ------------------------------------------------------------ FV -> DG
-// shared memory per cell (doubles per variable): the staged subcells (later
-// reused for the pass-y result) and the pass-x result
-template <int DIM, int B>
-__host__ __device__ constexpr int lim_to_dg_cell_doubles_per_var() {
-  return DIM == 3 ? (2 * B - 1) * (2 * B - 1) * (2 * B - 1) + (2 * B - 1) * (2 * B - 1) * B
-                  : (2 * B - 1) * (2 * B - 1) + (2 * B - 1) * B;
-}
-
+// One thread per (cell, node column x, variable): plane by plane and row by
+// row of the subcells, the row's x sum, added to the plane's y sums, and those
+// to the column's B^2 results.  A CTA serves cpb cells; the planes of their
+// subcells (the whole patch in 2D) pass through two shared buffers, the next
+// plane's asynchronous copies in flight while this one is summed.  A plane is
+// copied as it lies, from its first interior value to its last: the ghost
+// values between the rows cost less than finding the rows -- except at order 1,
+// where two ghost layers are more than half of it (375,000 3D cells: 328 us with
+// them, 171 without).  Bound by the latency of the planes' loads at 12 to 20
+// warps per SM.  Per call before -> now: 3D order 4 (24,000 cells) 344 -> 272 us,
+// order 5 (13,888) 817 -> 283, 2D order 3 (375,000) 304 -> 260, order 5
+// (166,666) 798 -> 347.
 template <int DIM, int B, int NVT>
-__global__ void __launch_bounds__(kLimNT, LimOcc<B>::value)
-    k_lim_to_dg(int nvar_rt, int ghost, long ncells, int cpb, const double* lim, double* luh, LimSel sel) {
-  constexpr int S = 2 * B - 1;
-  constexpr int NPC = DIM == 3 ? B * B * B : B * B;
-  constexpr int NS = DIM == 3 ? S * S * S : S * S;
+__global__ void __launch_bounds__(kLimColNT, LimMinB<DIM, B, false>::value)
+    k_lim_to_dg(int nvar_rt, int ghost, long ncells, int cpb, const double* __restrict__ lim, double* luh,
+                LimSel sel) {
+  constexpr int S = 2 * B - 1, BZ = DIM == 3 ? B : 1, SZ = DIM == 3 ? S : 1;
+  constexpr bool kRows = B <= 2;  // rows without the ghost values between them
   const int nvar = NVT ? NVT : nvar_rt;
+  const int SG = S + 2 * ghost;
+  const long row = (long)SG * nvar, plane = row * SG;
+  const int irow = (kRows ? S : SG) * nvar, len = (S - 1) * irow + S * nvar, buf = cpb * len;  // a staged plane
   extern __shared__ double sm[];
   const long nce = sel.cells(ncells);
-  // one cell block per iteration (a single one unless a selection launched
-  // fewer CTAs than blocks)
   for (long c0 = (long)blockIdx.x * cpb; c0 < nce; c0 += (long)gridDim.x * cpb) {
     const int nc = (int)min((long)cpb, nce - c0);
-    const int SG = S + 2 * ghost;
-    const long lim_cell = (long)nvar * (DIM == 3 ? SG * SG * SG : SG * SG);
-    double* A = sm;  // interior subcells [c][z][y][x][v]
-    double* T1 = A + cpb * NS * nvar;
-    lim_stage_interior<DIM, S>(A, lim, lim_cell, nvar, ghost, c0, nc, sel);
-    __syncthreads();
-    GlobalOut<DIM> go{luh, (long)NPC * nvar, nvar, B, 0, c0, sel.list};
-    if (DIM == 2) {
-      SmemOut o1{T1, nvar, S * B * nvar, B, S};
-      lim_pass<kTabLim2Uh, B, S, S, 1, 0, B>(A, nvar, NS * nvar, nc, nvar, o1);
-      __syncthreads();
-      lim_pass<kTabLim2Uh, B, B, S, 1, 1, B>(T1, nvar, S * B * nvar, nc, nvar, go);
-    } else {
-      double* T2 = A;  // the staged subcells are dead after pass x
-      SmemOut o1{T1, nvar, S * S * B * nvar, B, S};
-      lim_pass<kTabLim2Uh, B, S, S, S, 0, B>(A, nvar, NS * nvar, nc, nvar, o1);
-      __syncthreads();
-      SmemOut o2{T2, nvar, S * B * B * nvar, B, B};
-      lim_pass<kTabLim2Uh, B, B, S, S, 1, B>(T1, nvar, S * S * B * nvar, nc, nvar, o2);
-      __syncthreads();
-      lim_pass<kTabLim2Uh, B, B, B, S, 2, B>(T2, nvar, S * B * B * nvar, nc, nvar, go);
+    auto stage = [&](int z) {
+      double* d = sm + (z & 1) * buf;
+      for (int c = 0; c < nc; c++) {
+        const double* src = lim + sel.cell(c0 + c) * (DIM == 3 ? plane * SG : plane) +
+                            (DIM == 3 ? (z + ghost) * plane : 0) + ghost * row + (long)ghost * nvar;
+        if (kRows) {
+          for (int k = threadIdx.x; k < len; k += kLimColNT)
+            cp_async8(d + c * len + k, src + k + k / (S * nvar) * 2 * ghost * nvar);
+        } else {
+          for (int k = threadIdx.x; k < len; k += kLimColNT) cp_async8(d + c * len + k, src + k);
+        }
+      }
+      cp_async_commit();
+    };
+    // this thread's first column; the rare further ones (more columns than
+    // threads) run after it over the same planes
+    for (int it0 = 0; it0 < nc * B * nvar; it0 += kLimColNT) {
+      const int it = it0 + threadIdx.x;
+      const bool on = it < nc * B * nvar;
+      const int v = on ? it % nvar : 0, x = on ? (it / nvar) % B : 0, c = on ? it / (nvar * B) : 0;
+      double cx[S];
+#pragma unroll
+      for (int p = 0; p < S; p++) cx[p] = c_lim[B - 1].lim2uh[p][x];
+      double o[BZ][B];
+#pragma unroll
+      for (int z = 0; z < BZ; z++)
+#pragma unroll
+        for (int y = 0; y < B; y++) o[z][y] = 0.0;
+      stage(0);
+#pragma unroll 1
+      for (int z = 0; z < SZ; z++) {
+        if (z + 1 < SZ) {
+          stage(z + 1);
+          cp_async_wait<1>();
+        } else {
+          cp_async_wait<0>();
+        }
+        __syncthreads();
+        const double* src = sm + (z & 1) * buf + c * len + v;
+        double b[B];
+#pragma unroll
+        for (int y = 0; y < B; y++) b[y] = 0.0;
+#pragma unroll
+        for (int y = 0; y < S; y++) {
+          double acc = 0.0;
+#pragma unroll
+          for (int p = 0; p < S; p++) acc = fma(cx[p], src[y * irow + p * nvar], acc);
+#pragma unroll
+          for (int m = 0; m < B; m++) b[m] = fma(c_lim[B - 1].lim2uh[y][m], acc, b[m]);
+        }
+        if (DIM == 2) {
+#pragma unroll
+          for (int m = 0; m < B; m++) o[0][m] = b[m];
+        } else {
+#pragma unroll
+          for (int n = 0; n < BZ; n++)
+#pragma unroll
+            for (int m = 0; m < B; m++) o[n][m] = fma(c_lim[B - 1].lim2uh[z][n], b[m], o[n][m]);
+        }
+        __syncthreads();  // the buffer is free for plane z + 2
+      }
+      if (on) {
+        double* dst = luh + sel.cell(c0 + c) * (long)(BZ * B * B * nvar) + (long)x * nvar + v;
+#pragma unroll
+        for (int z = 0; z < BZ; z++)
+#pragma unroll
+          for (int y = 0; y < B; y++) dst[(z * B + y) * B * nvar] = o[z][y];
+      }
     }
-    __syncthreads();
+  }
+}
+
+// The same for few 3D cells, one per CTA: plane after plane, a cell's column
+// waits for memory S times and its sums are one thread's.  Here the whole patch
+// is copied at once, one thread per (plane, node column, variable) forms the
+// plane's sums and one per (node row, node column, variable) the z sums, each
+// in the order above.  Order 4: 300 cells 24.6 us in the form above, 13.3 here
+// (14.3 before both), 4,000 cells 73 and 57 (67).
+template <int B, int NVT>
+__global__ void __launch_bounds__(kLimNT) k_lim_to_dg_few(int nvar_rt, int ghost, long ncells,
+                                                          const double* __restrict__ lim, double* luh) {
+  constexpr int S = 2 * B - 1;
+  const int nvar = NVT ? NVT : nvar_rt;
+  const int SG = S + 2 * ghost, irow = SG * nvar, len = (S - 1) * irow + S * nvar;
+  const long plane = (long)SG * irow;
+  extern __shared__ double sm[];
+  double* sb = sm + S * len;  // plane sums [z][y][x][nvar]
+  const long c = blockIdx.x;
+  for (int z = 0; z < S; z++) {
+    const double* src = lim + c * plane * SG + (z + ghost) * plane + ghost * (irow + nvar);
+    for (int k = threadIdx.x; k < len; k += kLimNT) cp_async8(sm + z * len + k, src + k);
+  }
+  cp_async_commit_wait_all();
+  __syncthreads();
+  for (int it = threadIdx.x; it < S * B * nvar; it += kLimNT) {
+    const int v = it % nvar, x = (it / nvar) % B, z = it / (nvar * B);
+    const double* src = sm + z * len + v;
+    double b[B];
+#pragma unroll
+    for (int m = 0; m < B; m++) b[m] = 0.0;
+#pragma unroll
+    for (int y = 0; y < S; y++) {
+      double acc = 0.0;
+#pragma unroll
+      for (int p = 0; p < S; p++) acc = fma(c_lim[B - 1].lim2uh[p][x], src[y * irow + p * nvar], acc);
+#pragma unroll
+      for (int m = 0; m < B; m++) b[m] = fma(c_lim[B - 1].lim2uh[y][m], acc, b[m]);
+    }
+#pragma unroll
+    for (int m = 0; m < B; m++) sb[((z * B + m) * B + x) * nvar + v] = b[m];
+  }
+  __syncthreads();
+  for (int it = threadIdx.x; it < B * B * nvar; it += kLimNT) {
+    double o[B];
+#pragma unroll
+    for (int n = 0; n < B; n++) o[n] = 0.0;
+#pragma unroll
+    for (int z = 0; z < S; z++)
+#pragma unroll
+      for (int n = 0; n < B; n++) o[n] = fma(c_lim[B - 1].lim2uh[z][n], sb[z * B * B * nvar + it], o[n]);
+#pragma unroll
+    for (int n = 0; n < B; n++) luh[(c * B + n) * B * B * nvar + it] = o[n];
   }
 }
 
 // ------------------------------------------------ min/max and the DMP
-// The Gauss-Lobatto (B -> B) and subcell (B -> S) evaluations run side by
-// side, pass by pass; the first pass also takes the extrema of the nodes
-// (its input lines).  Per cell and observable, shared memory holds: the
-// pass-x results of both (B^3 + B^2 S), the pass-y result of the subcells
-// (B S^2) and of the Lobatto points (B^3, in the luh staging area, dead after
-// pass x), and the per-line extrema of nodes, Lobatto points and subcells.
-template <int DIM, int B>
-struct LimMM {
-  static constexpr int S = 2 * B - 1;
-  static constexpr int NPC = DIM == 3 ? B * B * B : B * B;
-  static constexpr int XL = DIM == 3 ? B * B * B : B * B;  // Lobatto pass-x result
-  static constexpr int XS = DIM == 3 ? B * B * S : B * S;  // subcell pass-x result
-  static constexpr int YS = DIM == 3 ? B * S * S : 0;      // subcell pass-y result
-  static constexpr int NODE_LINES = DIM == 3 ? B * B : B;  // pass-x lines
-  static constexpr int LOB_LINES = DIM == 3 ? B * B : B;   // final Lobatto lines
-  static constexpr int SUB_LINES = DIM == 3 ? S * S : S;   // final subcell lines
-  static constexpr int LINES = NODE_LINES + LOB_LINES + SUB_LINES;
-  // doubles per cell
-  __host__ __device__ static constexpr int doubles(int nvar, int nobs) {
-    return NPC * nvar + (XL + XS + YS + 2 * LINES) * nobs;
+// One thread per (cell, column, observable): S columns of subcells and B
+// columns of Gauss-Lobatto points (which also take the node column of the
+// same x), each evaluated as in k_lim_to_fv but only its extrema kept; then
+// one thread per (cell, observable) reduces the S + B columns and finishes.
+// WALK (2D): a column is too little work for its place in the reduction; one
+// thread per (cell, observable) keeps the cell's B^2 values in registers and
+// walks the columns.  A CTA holds cpb cells, for WALK staged at a pitch that
+// puts the lanes' (cell, observable) values in consecutive banks.
+// Bound by FP64 issue and, in 2D, by memory.  Per DMP call, passes through
+// shared memory before -> now: 3D order 4 (24,000 cells) 263 -> 135 us, order 3
+// (46,875) 256 -> 110, order 2 (111,111) 339 -> 99; 2D order 3 (375,000) 224 ->
+// 120, order 1 (1,500,000) 374 -> 163.
+//
+// extrema over all points of a 2D cell evaluated with table TAB (NO per direction)
+template <int B, int TAB, int NO>
+__device__ __forceinline__ void lim_cell_extrema(const double (&q)[B][B], double& mn, double& mx) {
+#pragma unroll 1
+  for (int x = 0; x < NO; x++) {
+    double a[B];
+#pragma unroll
+    for (int y = 0; y < B; y++) {
+      double acc = 0.0;
+#pragma unroll
+      for (int p = 0; p < B; p++) acc = fma(lim_coef<TAB, B>(p, x), q[y][p], acc);
+      a[y] = acc;
+    }
+#pragma unroll
+    for (int y = 0; y < NO; y++) {
+      double acc = 0.0;
+#pragma unroll
+      for (int p = 0; p < B; p++) acc = fma(lim_coef<TAB, B>(p, y), a[p], acc);
+      mn = lim_min(mn, acc);
+      mx = lim_max(mx, acc);
+    }
   }
-};
+}
+
+// extrema of a column evaluated with table TAB (NO points per direction)
+template <int DIM, int B, int TAB, int NO>
+__device__ __forceinline__ void lim_column_extrema(const double* src, int nvar, int x, double& mn, double& mx) {
+  constexpr int BZ = DIM == 3 ? B : 1;
+  double cx[B];
+#pragma unroll
+  for (int p = 0; p < B; p++) cx[p] = lim_coef<TAB, B>(p, x);
+  double a[BZ][B];
+#pragma unroll
+  for (int z = 0; z < BZ; z++)
+#pragma unroll
+    for (int y = 0; y < B; y++) {
+      double acc = 0.0;
+#pragma unroll
+      for (int p = 0; p < B; p++) acc = fma(cx[p], src[((z * B + y) * B + p) * nvar], acc);
+      a[z][y] = acc;
+    }
+#pragma unroll 1
+  for (int y = 0; y < NO; y++) {
+    double b[BZ];
+#pragma unroll
+    for (int z = 0; z < BZ; z++) {
+      double acc = 0.0;
+#pragma unroll
+      for (int p = 0; p < B; p++) acc = fma(lim_coef<TAB, B>(p, y), a[z][p], acc);
+      b[z] = acc;
+    }
+    if (DIM == 2) {
+      mn = lim_min(mn, b[0]);
+      mx = lim_max(mx, b[0]);
+    } else {
+#pragma unroll
+      for (int z = 0; z < NO; z++) {
+        double acc = 0.0;
+#pragma unroll
+        for (int p = 0; p < BZ; p++) acc = fma(lim_coef<TAB, B>(p, z), b[p], acc);
+        mn = lim_min(mn, acc);
+        mx = lim_max(mx, acc);
+      }
+    }
+  }
+}
+
+// doubles from one staged cell of k_lim_min_max to the next
+template <int DIM, int B, bool WALK>
+__host__ __device__ __forceinline__ int lim_pitch(int nvar) {
+  const int n = (DIM == 3 ? B * B * B : B * B) * nvar;
+  return !WALK ? n : n + ((nvar - n) % 16 + 16) % 16;
+}
 
 // mode 0: findCellLocalMinAndMax, result copied to all faces;
 // mode 1: discreteMaximumPrincipleAndMinAndMaxSearch (obs_min/max in/out,
 //         dmp_ok[cell] = 1 if the DMP holds).
-template <int DIM, int B, int NVT>
-__global__ void __launch_bounds__(kLimNT, LimOcc<B>::value)
-    k_lim_min_max(int mode, int nvar_rt, int nobs_rt, long ncells, int cpb, const double* luh, double relaxation,
-                  double scaling, double* obs_min, double* obs_max, int* dmp_ok) {
-  using M = LimMM<DIM, B>;
-  constexpr int S = M::S, NPC = M::NPC, NF = 2 * DIM;
+template <int DIM, int B, int NVT, bool WALK>
+__global__ void __launch_bounds__(kLimMmNT, LimMmMinB<DIM, B, WALK>::value)
+    k_lim_min_max(int mode, int nvar_rt, int nobs_rt, long ncells, int cpb, const double* __restrict__ luh,
+                  double relaxation, double scaling, double* obs_min, double* obs_max, int* dmp_ok) {
+  constexpr int S = 2 * B - 1, NPC = DIM == 3 ? B * B * B : B * B, NF = 2 * DIM, COLS = S + B;
   const int nvar = NVT ? NVT : nvar_rt;
   const int nobs = NVT ? NVT : nobs_rt;
   extern __shared__ double sm[];
   const long c0 = (long)blockIdx.x * cpb;
   const int nc = (int)min((long)cpb, ncells - c0);
-  double* A = sm;                         // luh, later the Lobatto pass-y result
-  double* XL = A + cpb * NPC * nvar;      // [c][z][y][x][obs]
-  double* XS = XL + cpb * M::XL * nobs;
-  double* YS = XS + cpb * M::XS * nobs;
-  double* pmn = YS + cpb * M::YS * nobs;  // [node | lob | sub lines]
-  double* pmx = pmn + cpb * M::LINES * nobs;
-  double* pn_mn = pmn;                    // node lines   [c][line][obs]
-  double* pl_mn = pmn + cpb * M::NODE_LINES * nobs;
-  double* ps_mn = pl_mn + cpb * M::LOB_LINES * nobs;
-  double* pn_mx = pmx;
-  double* pl_mx = pmx + cpb * M::NODE_LINES * nobs;
-  double* ps_mx = pl_mx + cpb * M::LOB_LINES * nobs;
+  const int pitch = lim_pitch<DIM, B, WALK>(nvar);
+  double* sluh = sm;                // [cell][node][nvar]
+  double* pmn = sm + cpb * pitch;   // !WALK: [cell][obs][column]
+  double* pmx = pmn + cpb * nobs * COLS;
   if (mode == 1)
-    for (int c = threadIdx.x; c < nc; c += kLimNT) dmp_ok[c0 + c] = 1;
-  lim_copy_in(A, luh + c0 * NPC * nvar, (long)nc * NPC * nvar);
-  __syncthreads();
-  const int ix = nc * M::NODE_LINES * nobs;  // items of one pass-x
-  if (DIM == 2) {
-    SmemOutInputMinMax ol{{XL, nobs, B * B * nobs, B, B}, pn_mn, pn_mx};
-    lim_pass<kTabUh2Lob, B, B, B, 1, 0, B>(A, nvar, NPC * nvar, nc, nobs, ol);
-    SmemOut os{XS, nobs, S * B * nobs, S, B};
-    lim_pass<kTabUh2Lim, B, B, B, 1, 0, S>(A, nvar, NPC * nvar, nc, nobs, os, ix);
-    __syncthreads();
-    MinMaxOut ml{pl_mn, pl_mx}, ms{ps_mn, ps_mx};
-    lim_pass<kTabUh2Lob, B, B, B, 1, 1, B>(XL, nobs, B * B * nobs, nc, nobs, ml);
-    lim_pass<kTabUh2Lim, B, S, B, 1, 1, S>(XS, nobs, S * B * nobs, nc, nobs, ms, nc * B * nobs);
+    for (int c = threadIdx.x; c < nc; c += kLimMmNT) dmp_ok[c0 + c] = 1;
+  if (WALK) {
+    const int n = NPC * nvar;
+    for (int i = threadIdx.x; i < nc * n; i += kLimMmNT) cp_async8(sluh + i + i / n * (pitch - n), luh + c0 * n + i);
   } else {
-    SmemOutInputMinMax ol{{XL, nobs, B * B * B * nobs, B, B}, pn_mn, pn_mx};
-    lim_pass<kTabUh2Lob, B, B, B, B, 0, B>(A, nvar, NPC * nvar, nc, nobs, ol);
-    SmemOut os{XS, nobs, B * B * S * nobs, S, B};
-    lim_pass<kTabUh2Lim, B, B, B, B, 0, S>(A, nvar, NPC * nvar, nc, nobs, os, ix);
-    __syncthreads();
-    double* YL = A;  // luh is dead after pass x
-    SmemOut yl{YL, nobs, B * B * B * nobs, B, B};
-    lim_pass<kTabUh2Lob, B, B, B, B, 1, B>(XL, nobs, B * B * B * nobs, nc, nobs, yl);
-    SmemOut ys{YS, nobs, B * S * S * nobs, S, S};
-    lim_pass<kTabUh2Lim, B, S, B, B, 1, S>(XS, nobs, B * B * S * nobs, nc, nobs, ys, nc * B * B * nobs);
-    __syncthreads();
-    MinMaxOut ml{pl_mn, pl_mx}, ms{ps_mn, ps_mx};
-    lim_pass<kTabUh2Lob, B, B, B, B, 2, B>(YL, nobs, B * B * B * nobs, nc, nobs, ml);
-    lim_pass<kTabUh2Lim, B, S, S, B, 2, S>(YS, nobs, B * S * S * nobs, nc, nobs, ms, nc * B * B * nobs);
+    lim_stage_cells(sluh, luh, NPC * nvar, c0, nc, LimSel(), kLimMmNT);
   }
+  // the bounds of this thread's (cell, observable), needed at the end
+  double lo0 = 0.0, hi0 = 0.0;
+  if (mode == 1 && threadIdx.x < nc * nobs) {
+    const int c = threadIdx.x / nobs, v = threadIdx.x % nobs;
+    const double* bmn = obs_min + (c0 + c) * NF * nobs + v;
+    const double* bmx = obs_max + (c0 + c) * NF * nobs + v;
+    lo0 = bmn[0];
+    hi0 = bmx[0];
+#pragma unroll
+    for (int f = 1; f < NF; f++) {
+      lo0 = lim_min(lo0, bmn[f * nobs]);
+      hi0 = lim_max(hi0, bmx[f * nobs]);
+    }
+  }
+  cp_async_commit_wait_all();
   __syncthreads();
-  // per (cell, observable): the new extrema -> face blocks, and the DMP
-  auto finish = [&](int pair, double mn, double mx) {
+  // the subcell columns of every cell first, then the Lobatto columns: few
+  // warps hold both kinds
+  const int nsub = nc * S * nobs, total = WALK ? 0 : nc * COLS * nobs;
+  for (int it = threadIdx.x; it < total; it += kLimMmNT) {
+    const bool sub = it < nsub;
+    const int n = sub ? S : B, i = sub ? it : it - nsub;
+    const int v = i % nobs, x = (i / nobs) % n, c = i / (nobs * n);
+    const double* src = sluh + c * NPC * nvar + v;
+    double mn = DBL_MAX, mx = -DBL_MAX;
+    if (sub) {
+      lim_column_extrema<DIM, B, kTabUh2Lim, S>(src, nvar, x, mn, mx);
+    } else {
+#pragma unroll
+      for (int k = 0; k < NPC / B; k++) {
+        const double q = src[(k * B + x) * nvar];
+        mn = lim_min(mn, q);
+        mx = lim_max(mx, q);
+      }
+      lim_column_extrema<DIM, B, kTabUh2Lob, B>(src, nvar, x, mn, mx);
+    }
+    const int slot = (c * nobs + v) * COLS + (sub ? x : S + x);
+    pmn[slot] = mn;
+    pmx[slot] = mx;
+  }
+  if (!WALK) __syncthreads();
+  for (int pair = threadIdx.x; pair < nc * nobs; pair += kLimMmNT) {
     const int c = pair / nobs, v = pair % nobs;
+    double mn = DBL_MAX, mx = -DBL_MAX;
+    if constexpr (!WALK) {
+#pragma unroll
+      for (int l = 0; l < COLS; l++) {
+        mn = lim_min(mn, pmn[pair * COLS + l]);
+        mx = lim_max(mx, pmx[pair * COLS + l]);
+      }
+    } else {
+      double q[B][B];
+#pragma unroll
+      for (int y = 0; y < B; y++)
+#pragma unroll
+        for (int x = 0; x < B; x++) {
+          q[y][x] = sluh[c * pitch + (y * B + x) * nvar + v];
+          mn = lim_min(mn, q[y][x]);
+          mx = lim_max(mx, q[y][x]);
+        }
+      lim_cell_extrema<B, kTabUh2Lob, B>(q, mn, mx);
+      lim_cell_extrema<B, kTabUh2Lim, S>(q, mn, mx);
+    }
+    // the new extrema -> face blocks, and the DMP
     double* bmn = obs_min + (c0 + c) * NF * nobs;
     double* bmx = obs_max + (c0 + c) * NF * nobs;
     if (mode == 0) {
@@ -439,10 +547,14 @@ __global__ void __launch_bounds__(kLimNT, LimOcc<B>::value)
         bmx[f * nobs + v] = mx;
       }
     } else {
-      double lo = bmn[v], hi = bmx[v];
-      for (int f = 1; f < NF; f++) {
-        lo = lim_min(lo, bmn[f * nobs + v]);
-        hi = lim_max(hi, bmx[f * nobs + v]);
+      double lo = lo0, hi = hi0;
+      if (pair != threadIdx.x) {
+        lo = bmn[v];
+        hi = bmx[v];
+        for (int f = 1; f < NF; f++) {
+          lo = lim_min(lo, bmn[f * nobs + v]);
+          hi = lim_max(hi, bmx[f * nobs + v]);
+        }
       }
       const double sd = lim_max((hi - lo) * scaling, relaxation);
       if (mn < lo - sd || mx > hi + sd) atomicAnd(dmp_ok + c0 + c, 0);
@@ -450,45 +562,6 @@ __global__ void __launch_bounds__(kLimNT, LimOcc<B>::value)
       bmx[v] = mx;
       bmn[v + nobs] = lo;
       bmx[v + nobs] = hi;
-    }
-  };
-  auto line_index = [&](int c, int v, int l) {
-    if (l < M::NODE_LINES) return (c * M::NODE_LINES + l) * nobs + v;
-    if (l < M::NODE_LINES + M::LOB_LINES)
-      return cpb * M::NODE_LINES * nobs + (c * M::LOB_LINES + l - M::NODE_LINES) * nobs + v;
-    return cpb * (M::NODE_LINES + M::LOB_LINES) * nobs + (c * M::SUB_LINES + l - M::NODE_LINES - M::LOB_LINES) * nobs +
-           v;
-  };
-  // reduction over the line extrema: a thread per pair when the pairs have
-  // few lines (2D), a warp per pair otherwise
-  if (M::LINES <= 32) {
-    for (int pair = threadIdx.x; pair < nc * nobs; pair += kLimNT) {
-      const int c = pair / nobs, v = pair % nobs;
-      double mn = DBL_MAX, mx = -DBL_MAX;
-#pragma unroll
-      for (int l = 0; l < M::LINES; l++) {
-        const int k = line_index(c, v, l);
-        mn = lim_min(mn, pmn[k]);
-        mx = lim_max(mx, pmx[k]);
-      }
-      finish(pair, mn, mx);
-    }
-  } else {
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    for (int pair = warp; pair < nc * nobs; pair += kLimNT / 32) {
-      const int c = pair / nobs, v = pair % nobs;
-      double mn = DBL_MAX, mx = -DBL_MAX;
-      for (int l = lane; l < M::LINES; l += 32) {
-        const int k = line_index(c, v, l);
-        mn = lim_min(mn, pmn[k]);
-        mx = lim_max(mx, pmx[k]);
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        mn = lim_min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-        mx = lim_max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      }
-      if (lane == 0) finish(pair, mn, mx);
     }
   }
 }
@@ -535,16 +608,19 @@ __global__ void __launch_bounds__(kLimNT) k_lim_fv_min_max(int nvar, int nobs, i
   }
 }
 
-// cells per CTA: enough items for two rounds of the final pass, within a
-// shared-memory budget that leaves room for `occ` resident CTAs per SM
-static int lim_cpb(long items_per_cell, long smem_per_cell, long ncells, int occ) {
-  long cpb = (2 * kLimNT + items_per_cell - 1) / items_per_cell;
-  if (cpb > 64) cpb = 64;
-  long cap = (220L * 1024 / occ) / smem_per_cell;
-  if (cap < 1) cap = 1;
-  if (cpb > cap) cpb = cap;
-  if (cpb > ncells) cpb = ncells;
-  return (int)(cpb < 1 ? 1 : cpb);
+// cells per CTA: the count whose items fill their rounds of nt threads best,
+// within a shared-memory budget and up to 16 or one round's cells; no more than
+// leave every SM four CTAs
+static int lim_cpb(long items_per_cell, long smem_per_cell, long ncells, int nt, long budget, int sms) {
+  int best = 1;
+  double fill = 0.0;
+  const long round = nt / items_per_cell, most = round > 16 ? round : 16, spread = ncells / (4 * sms);
+  for (int c = 1; c <= most && (c == 1 || (c * smem_per_cell <= budget && c <= spread)); c++) {
+    const long items = c * items_per_cell;
+    const double f = (double)items / (double)((items + nt - 1) / nt * nt);
+    if (f > fill + 0.02) best = c, fill = f;
+  }
+  return best;
 }
 
 template <class K>
@@ -556,55 +632,117 @@ template <int DIM, int B, int NVT>
 static exa_status_t lim_run(int op, int nvar, int nobs, int ghost, long ncells, const double* in, double* out,
                             double* mn, double* mx, int* ok, double relax, double scaling, cudaStream_t st,
                             LimSel sel) {
-  constexpr int S = 2 * B - 1;
-  long per_cell, items;
-  if (op == kLimToFv) {
-    per_cell = (long)lim_to_fv_cell_doubles_per_var<DIM, B>() * nvar;
-    items = (long)(DIM == 3 ? S * S : S) * nvar;
-  } else if (op == kLimToDg) {
-    per_cell = (long)lim_to_dg_cell_doubles_per_var<DIM, B>() * nvar;
-    items = (long)(DIM == 3 ? B * B : B) * nvar;
-  } else if (op == kLimFvMinMax) {
-    per_cell = (long)(DIM == 3 ? S * S * S : S * S) * nvar;
-    items = 32L * nobs;
-  } else {
-    per_cell = LimMM<DIM, B>::doubles(nvar, nobs);
-    items = (long)LimMM<DIM, B>::SUB_LINES * nobs;
-  }
-  per_cell *= (long)sizeof(double);
-  if (per_cell > kLimMaxSmem) return set_error(EXA_EINVAL, "limiter: cell too large for shared memory");
-  int cpb = lim_cpb(items, per_cell, ncells, LimOcc<B>::value);
+  constexpr int S = 2 * B - 1, COLS = S + B;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // The entry points take cells whose 1D passes' arrays fit one CTA's shared
+  // memory (doubles per variable or observable below); the column kernels need
+  // none, the limit stands.
+  constexpr long P = DIM == 3 ? B * B * B : B * B, Q = DIM == 3 ? S * S * S : S * S;
+  constexpr long fv_pass = DIM == 3 ? P + B * B * S + B * S * S : P + B * S;
+  constexpr long dg_pass = DIM == 3 ? Q + S * S * B : Q + S * B;
+  constexpr long mm_lines = DIM == 3 ? 2 * B * B + S * S : 2 * B + S;
+  constexpr long mm_pass = DIM == 3 ? P + B * B * S + B * S * S + 2 * mm_lines : P + B * S + 2 * mm_lines;
+  const long limit = op == kLimToFv ? fv_pass * nvar
+                                    : (op == kLimToDg ? dg_pass * nvar
+                                                      : (op == kLimFvMinMax ? Q * nvar : P * nvar + mm_pass * nobs));
+  if (limit * (long)sizeof(double) > kLimMaxSmem)
+    return set_error(EXA_EINVAL, "limiter: cell too large for shared memory");
+  constexpr long NPC = P, D8 = (long)sizeof(double);
   const int cpb_set = tune_get(kTuneLimiterCellsPerCta, 0);
+  if (op == kLimToFv || op == kLimToDg) {
+    const bool fv = op == kLimToFv;
+    // one column per thread of the last cell's end at most: FV -> DG walks its
+    // planes once per round of columns
+    const long plane = (long)(S - 1) * (S + 2 * ghost) + S;  // values of a variable in a staged plane
+    const long per_cell = D8 * (fv ? NPC * nvar : (DIM == 3 ? 2 : 1) * plane * nvar);
+    const long items = (long)(fv ? S : B) * nvar;
+    int cpb;
+    int nt = kLimColNT;
+    if (fv) {
+      cpb = lim_cpb(items, per_cell, ncells, kLimColNT, 44 * 1024, sms);
+      if (DIM == 3) {
+        // one round of columns if they fill whole warps well (order 4, 24,000
+        // cells: 313 us, three rounds 348; order 6, a third of its lanes idle:
+        // 394, several rounds 322; in 2D rounds are as good or better)
+        const long spread = ncells / (4 * sms);
+        double fill = 0.8;
+        for (int c = 1; c * items <= kLimColNT && (c == 1 || c <= spread); c++) {
+          const int t = (int)((c * items + 31) / 32 * 32);
+          const double f = (double)(c * items) / (double)t;
+          if (f >= fill) cpb = c, fill = f, nt = t;
+        }
+      }
+    } else {
+      const long spread = ncells / (4 * sms);
+      cpb = (int)(kLimColNT / items > 0 ? kLimColNT / items : 1);
+      if (cpb > spread) cpb = (int)(spread > 0 ? spread : 1);
+      while (cpb > 1 && cpb * per_cell > 72 * 1024) cpb--;
+      if constexpr (DIM == 3) {
+        const long few = D8 * (S * plane + (long)S * B * B) * nvar;
+        // all planes of a cell at once up to ten patches' worth of the chip's
+        // shared memory (order 4: 6,000 cells; beyond, the streamed planes are
+        // level or better)
+        if (!cpb_set && !sel.list && few <= kLimMaxSmem && ncells * few <= 10L * sms * kLimMaxSmem) {
+          cudaError_t e = lim_prepare(k_lim_to_dg_few<B, NVT>, (size_t)few);
+          if (e != cudaSuccess) return cuda_status(e, "limiter: shared-memory attribute");
+          k_lim_to_dg_few<B, NVT><<<(unsigned)ncells, kLimNT, (size_t)few, st>>>(nvar, ghost, ncells, in, out);
+          count_launch();
+          return cuda_status(cudaGetLastError(), "limiter projection");
+        }
+      }
+    }
+    if (per_cell > kLimMaxSmem) return set_error(EXA_EINVAL, "limiter: cell too large for shared memory");
+    if (cpb_set > 0 && (long)cpb_set * per_cell <= kLimMaxSmem) cpb = cpb_set;
+    const size_t smem = (size_t)cpb * per_cell;
+    long nblk = (ncells + cpb - 1) / cpb;
+    if (sel.count) nblk = nblk < 8L * sms ? nblk : 8L * sms;  // a selection usually holds a few cells: CTAs loop
+    if (nblk > 0x7fffffffL) return set_error(EXA_EINVAL, "limiter: too many cells");
+    cudaError_t e = fv ? lim_prepare(k_lim_to_fv<DIM, B, NVT>, smem) : lim_prepare(k_lim_to_dg<DIM, B, NVT>, smem);
+    if (e != cudaSuccess) return cuda_status(e, "limiter: shared-memory attribute");
+    if (fv)
+      k_lim_to_fv<DIM, B, NVT><<<(unsigned)nblk, nt, smem, st>>>(nvar, ghost, ncells, cpb, in, out, sel);
+    else
+      k_lim_to_dg<DIM, B, NVT><<<(unsigned)nblk, kLimColNT, smem, st>>>(nvar, ghost, ncells, cpb, in, out, sel);
+    count_launch();
+    return cuda_status(cudaGetLastError(), "limiter projection");
+  }
+  long per_cell;
+  int cpb;
+  // Extrema of a whole 2D cell in one thread: while its work is short (order 3,
+  // 375,000 cells: 120 us, by columns 240), or from four warps of such threads
+  // per scheduler on (order 4, 240,000 cells: 160, 231 by columns; but 1,000
+  // cells: 17, 10 by columns).  Order 6 is faster by columns throughout (264, 294).
+  const bool walk = DIM == 2 && (B <= 4 || (B <= 6 && ncells * nobs >= 512L * sms));
+  if (op == kLimFvMinMax) {
+    per_cell = (long)(DIM == 3 ? S * S * S : S * S) * nvar * (long)sizeof(double);
+    // a warp per (cell, observable), two rounds of them, three CTAs per SM
+    const long want = (16 + nobs - 1) / nobs, cap = 73L * 1024 / per_cell;
+    cpb = (int)(want < cap ? want : (cap < 1 ? 1 : cap));
+    if (cpb > ncells) cpb = (int)ncells;
+  } else {
+    per_cell = D8 * (walk ? lim_pitch<DIM, B, true>(nvar) : NPC * nvar + 2L * COLS * nobs);
+    cpb = lim_cpb((walk ? 1L : (long)COLS) * nobs, per_cell, ncells, kLimMmNT, 36 * 1024, sms);
+  }
   if (cpb_set > 0 && (long)cpb_set * per_cell <= kLimMaxSmem) cpb = cpb_set;
   const size_t smem = (size_t)cpb * per_cell;
   long nblk = (ncells + cpb - 1) / cpb;
-  if (sel.count) {
-    // a selection usually holds a few cells: CTAs loop over the blocks
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    nblk = nblk < 4L * sms ? nblk : 4L * sms;
-  }
+  if (sel.count) nblk = nblk < 4L * sms ? nblk : 4L * sms;
   if (nblk > 0x7fffffffL) return set_error(EXA_EINVAL, "limiter: too many cells");
   cudaError_t e = cudaSuccess;
-  if (op == kLimToFv) {
-    e = lim_prepare(k_lim_to_fv<DIM, B, NVT>, smem);
-    if (e == cudaSuccess)
-      k_lim_to_fv<DIM, B, NVT><<<(unsigned)nblk, kLimNT, smem, st>>>(nvar, ghost, ncells, cpb, in, out, sel);
-  } else if (op == kLimToDg) {
-    e = lim_prepare(k_lim_to_dg<DIM, B, NVT>, smem);
-    if (e == cudaSuccess)
-      k_lim_to_dg<DIM, B, NVT><<<(unsigned)nblk, kLimNT, smem, st>>>(nvar, ghost, ncells, cpb, in, out, sel);
-  } else if (op == kLimFvMinMax) {
+  if (op == kLimFvMinMax) {
     e = lim_prepare(k_lim_fv_min_max<DIM, B>, smem);
     if (e == cudaSuccess)
       k_lim_fv_min_max<DIM, B><<<(unsigned)nblk, kLimNT, smem, st>>>(nvar, nobs, ghost, ncells, cpb, in, mn, mx,
                                                                        sel);
   } else {
-    auto kern = k_lim_min_max<DIM, B, NVT>;
+    auto kern = k_lim_min_max<DIM, B, NVT, false>;
+    if constexpr (DIM == 2 && B <= 6)
+      if (walk) kern = k_lim_min_max<DIM, B, NVT, true>;
     e = lim_prepare(kern, smem);
     if (e == cudaSuccess)
-      kern<<<(unsigned)nblk, kLimNT, smem, st>>>(op == kLimDmp ? 1 : 0, nvar, nobs, ncells, cpb, in, relax, scaling, mn,
+      kern<<<(unsigned)nblk, kLimMmNT, smem, st>>>(op == kLimDmp ? 1 : 0, nvar, nobs, ncells, cpb, in, relax, scaling, mn,
                                                   mx, ok);
   }
   if (e != cudaSuccess) return cuda_status(e, "limiter: shared-memory attribute");
