@@ -9,11 +9,11 @@
 //                      Troubled stay so for steps-till-cured more steps, then
 //                      become NeighbourOfTroubled1 (determineLimiterStatus-
 //                      AfterSolutionUpdate, :933-991)
-//   k_lim_spread       one face-neighbour hop of status spreading: a cell
-//                      takes max(own, neighbour - 1) (ADERDGSolver.cpp
-//                      mergeWithLimiterStatus :2482-2500)
-//   k_lim_lists        the cells that need a subcell patch (status >=
-//                      NeighbourOfTroubled3) and the cells the FV solver
+//   k_lim_spread       two face-neighbour hops of status spreading: with each
+//                      hop a cell takes max(own, neighbour - 1) (ADERDGSolver.cpp
+//                      mergeWithLimiterStatus :2482-2500); the second launch
+//                      also lists the cells that need a subcell patch (status
+//                      >= NeighbourOfTroubled3) and the cells the FV solver
 //                      updates (status >= NeighbourOfTroubled2)
 //   k_lim_local /      the new cell-local extrema and their merge with the
 //   k_lim_merge        face neighbours' (mergeSolutionMinMaxOnFace,
@@ -38,8 +38,11 @@ __global__ void k_lim_admissible(int npc, long ncells, int planar, const double*
   if (!(rho > 0.0 && p > 0.0 && isfinite(p))) ok[i / npc] = 0;
 }
 
-__global__ void k_lim_base_status(long ncells, const int* ok, int* status, int* cure, int steps_till_cured) {
+// also clears the counters that the listing adds to
+__global__ void k_lim_base_status(long ncells, const int* ok, int* status, int* cure, int steps_till_cured,
+                                  int* counts) {
   const long c = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c < 3) counts[c] = 0;
   if (c >= ncells) return;
   int base = 0;
   if (!ok[c]) {
@@ -64,9 +67,17 @@ struct LimGrid {
   int nx, ny, nz, dim;
   int bc[3];
   __host__ __device__ __forceinline__ long cells() const { return (long)nx * ny * nz; }
+  // (32-bit divisions: the cells are far below 2^31)
+  __device__ __forceinline__ void coords(long c, int& x, int& y, int& z) const {
+    const unsigned row = (unsigned)c / (unsigned)nx;
+    x = (int)((unsigned)c - row * (unsigned)nx);
+    z = (int)(row / (unsigned)ny);
+    y = (int)row - z * ny;
+  }
   // the neighbour across face f = 2 d + (0 lower, 1 upper), -1 outside
   __device__ __forceinline__ long nb(long c, int f) const {
-    int x = (int)(c % nx), y = (int)((c / nx) % ny), z = (int)(c / ((long)nx * ny));
+    int x, y, z;
+    coords(c, x, y, z);
     const int d = f >> 1;
     const bool up = f & 1;
     int* p = d == 0 ? &x : (d == 1 ? &y : &z);
@@ -81,26 +92,44 @@ struct LimGrid {
   }
 };
 
-__global__ void k_lim_spread(LimGrid G, const int* in, int* out) {
+// Two hops at once: the largest in[cell'] - k over the cells at face distance
+// k <= 2 (in a box, walls or not, k is |dx| + |dy| + |dz|).  One hop per launch
+// took four launches of 5 us for 59,049 cells and a memset and a launch for the
+// lists; the launches, not their work, were the cost.
+// LISTS: counts[0]: cells with a subcell patch, counts[1]: FV-updated cells,
+// counts[2]: Troubled cells
+template <bool LISTS>
+__global__ void k_lim_spread(LimGrid G, const int* in, int* out, int* list_patch, int* list_fv, int* counts) {
   const long c = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= G.cells()) return;
-  int nb = 0;
-  for (int f = 0; f < 2 * G.dim; f++) {
-    const long o = G.nb(c, f);
-    if (o >= 0) nb = max(nb, in[o]);
+  int x, y, z;
+  G.coords(c, x, y, z);
+  auto fold = [](int i, int n, int rule) {  // -1: outside the domain
+    if (i >= 0 && i < n) return i;
+    return rule != 0 ? -1 : (i % n + n) % n;
+  };
+  const int rz = G.dim == 3 ? 2 : 0;
+  int s = 0;
+  for (int dz = -rz; dz <= rz; dz++) {
+    const int zz = fold(z + dz, G.nz, G.bc[2]);
+    if (zz < 0) continue;
+    const int ry = 2 - abs(dz);
+    for (int dy = -ry; dy <= ry; dy++) {
+      const int yy = fold(y + dy, G.ny, G.bc[1]);
+      if (yy < 0) continue;
+      const int rx = ry - abs(dy);
+      for (int dx = -rx; dx <= rx; dx++) {
+        const int xx = fold(x + dx, G.nx, G.bc[0]);
+        if (xx >= 0) s = max(s, in[((long)zz * G.ny + yy) * G.nx + xx] - (abs(dx) + abs(dy) + abs(dz)));
+      }
+    }
   }
-  out[c] = max(in[c], nb - 1);
-}
-
-// counts[0]: cells with a subcell patch, counts[1]: FV-updated cells,
-// counts[2]: Troubled cells
-__global__ void k_lim_lists(long ncells, const int* status, int* list_patch, int* list_fv, int* counts) {
-  const long c = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncells) return;
-  const int s = status[c];
-  if (s >= kLimNT3) list_patch[atomicAdd(counts + 0, 1)] = (int)c;
-  if (s >= kLimNT2) list_fv[atomicAdd(counts + 1, 1)] = (int)c;
-  if (s == kLimTroubled) atomicAdd(counts + 2, 1);
+  out[c] = s;
+  if (LISTS) {
+    if (s >= kLimNT3) list_patch[atomicAdd(counts + 0, 1)] = (int)c;
+    if (s >= kLimNT2) list_fv[atomicAdd(counts + 1, 1)] = (int)c;
+    if (s == kLimTroubled) atomicAdd(counts + 2, 1);
+  }
 }
 
 // face block 0 of the per-cell extrema -> loc [cell][min | max][nobs]
@@ -158,15 +187,12 @@ exa_status_t limiting_status(int dim, const int* ncell, const int* bc, int npc, 
   const LimGrid G = lim_grid(dim, ncell, bc);
   const long n = (long)G.nx * G.ny * G.nz;
   if (admissibility) k_lim_admissible<<<blocks(n * npc, 256), 256, 0, st>>>(npc, n, planar, luh, ok);
-  k_lim_base_status<<<blocks(n, 256), 256, 0, st>>>(n, ok, status, cure, steps_till_cured);
+  // (a grid of one or two cells still has the threads that clear the counters)
+  k_lim_base_status<<<blocks(n, 256), 256, 0, st>>>(n, ok, status, cure, steps_till_cured, counts);
   // four hops: Troubled (5) reaches NeighbourOfTroubled4 (1)
-  for (int h = 0; h < 4; h++) {
-    k_lim_spread<<<blocks(n, 256), 256, 0, st>>>(G, (h & 1) ? status_tmp : status, (h & 1) ? status : status_tmp);
-  }
-  cudaError_t e = cudaMemsetAsync(counts, 0, 3 * sizeof(int), st);
-  if (e != cudaSuccess) return cuda_status(e, "limiter counters");
-  k_lim_lists<<<blocks(n, 256), 256, 0, st>>>(n, status, list_patch, list_fv, counts);
-  count_launch(6 + (admissibility ? 1 : 0));
+  k_lim_spread<false><<<blocks(n, 256), 256, 0, st>>>(G, status, status_tmp, nullptr, nullptr, nullptr);
+  k_lim_spread<true><<<blocks(n, 256), 256, 0, st>>>(G, status_tmp, status, list_patch, list_fv, counts);
+  count_launch(3 + (admissibility ? 1 : 0));
   return cuda_status(cudaGetLastError(), "limiter status kernels");
 }
 
