@@ -44,6 +44,7 @@ struct FVArgs {
   // fused steps: a grid of npx x npy patches (one patch: 1 x 1) and its
   // boundary rule per dimension (EXA_BC_*)
   int npx, npy, bcx, bcy;
+  int rows;  // Godunov sweep: rows of a strip
 };
 
 // Periodic index of a cell coordinate of a single patch with ghost width g:
@@ -101,6 +102,26 @@ __device__ __forceinline__ long fv_stencil_offset(const FVArgs& a, int X, int Y,
 // Per cell-update HBM traffic: one state read, one state write.
 
 
+// Pressure, sound speed, flux and largest |eigenvalue| of a cell for the Godunov
+// kernels, with every multiply-add written out: a sum of two products may be
+// fused either way round, and the sweeps and the tile kernel are to give the
+// same bits.
+template <bool PLANAR>
+struct FVPoint {
+  double irho, p, c;
+  __device__ __forceinline__ explicit FVPoint(const double* q) {
+    irho = 1.0 / q[0];
+    double j2 = fma(q[2], q[2], __dmul_rn(q[1], q[1]));
+    if (!PLANAR) j2 = fma(q[3], q[3], j2);
+    p = __dmul_rn(kGamma - 1.0, fma(-0.5 * j2, irho, q[4]));
+    c = sqrt(__dmul_rn(__dmul_rn(kGamma, p), irho));
+  }
+  __device__ __forceinline__ double max_eig(const double* q, int d) const {
+    const double un = __dmul_rn(q[d + 1], irho);
+    return fmax(fabs(__dadd_rn(un, -c)), fmax(fabs(un), fabs(__dadd_rn(un, c))));
+  }
+};
+
 // The next step's CFL dt over the cells a warp updated: the minimum over
 // its cells and both directions of 0.45 h_d / s_d (s_d the cell's largest
 // |eigenvalue| in direction d, commons::stableTimeStepSize), taken as
@@ -113,8 +134,9 @@ struct FVNextDt {
   double sx = 0.0, sy = 0.0;
   template <bool PLANAR>
   __device__ __forceinline__ void add(const double* u) {
-    sx = fmax(sx, euler_max_eig<PLANAR>(u, 0));
-    sy = fmax(sy, euler_max_eig<PLANAR>(u, 1));
+    const FVPoint<PLANAR> e(u);
+    sx = fmax(sx, e.max_eig(u, 0));
+    sy = fmax(sy, e.max_eig(u, 1));
   }
   // every lane of the warp calls it; lane 0 reduces into slot
   __device__ __forceinline__ void commit(const FVArgs& a, unsigned long long* slot, bool lane0) {
@@ -152,11 +174,13 @@ __device__ __forceinline__ double rusanov(const double* qL, const double* qR, in
 // so every face flux is the same value.
 template <bool PLANAR>
 __device__ __forceinline__ void fv_cell_flux(const double* q, int d, double* out) {
-  double F[2][kV];
-  euler_flux<2, PLANAR>(q, F);
+  const FVPoint<PLANAR> e(q);
+  const double ij = __dmul_rn(q[d + 1], e.irho);
+  out[0] = q[d + 1];
 #pragma unroll
-  for (int m = 0; m < kV; m++) out[m] = F[d][m];
-  out[kV] = euler_max_eig<PLANAR>(q, d);
+  for (int m = 1; m < 4; m++) out[m] = m == d + 1 ? fma(ij, q[m], e.p) : __dmul_rn(ij, q[m]);
+  out[4] = __dmul_rn(ij, __dadd_rn(q[4], e.p));
+  out[kV] = e.max_eig(q, d);
 }
 
 // rusanov() from per-cell fluxes: cl/cr = [F_d(q), lambda] of the left and
@@ -166,9 +190,7 @@ __device__ __forceinline__ double fv_face_flux(const double* qL, const double* q
   const double smax = fmax(cl[kV], cr[kV]);
 #pragma unroll
   for (int i = 0; i < kV; i++) {
-    double v = 0.5 * smax * (qL[i] - qR[i]);
-    v += 0.5 * (cl[i] + cr[i]);
-    f[i] = v;
+    f[i] = fma(0.5 * smax, __dadd_rn(qL[i], -qR[i]), 0.5 * __dadd_rn(cl[i], cr[i]));
   }
   return smax;
 }
@@ -179,7 +201,7 @@ __device__ __forceinline__ double fv_face_flux(const double* qL, const double* q
 // / a.out (the body of k_fv_godunov; the serving batch calls it per entry).
 // Godunov step as a sweep in y (one periodic patch, or the global view of a
 // patch grid): each warp owns a strip of FVS_W output columns (lane l =
-// column k0 - 1 + l; lanes 0 and 31 are halo columns) and walks up FVS_H
+// column k0 - 1 + l; lanes 0 and 31 are halo columns) and walks up a.rows
 // rows.  A lane loads its cell of the next row into registers, evaluates F_x,
 // F_y and their eigenvalue bounds once, takes the left neighbour's x values
 // by a warp shuffle and the row below's y values from its own registers, so
@@ -188,13 +210,37 @@ __device__ __forceinline__ double fv_face_flux(const double* qL, const double* q
 // the row above is known), bit for bit.
 constexpr int FVS_W = 30, FVS_WARPS = 4, FVS_H = 32;
 
+// Rows of a strip, at most FVS_H.  A strip is one chain of loads and solves over
+// its rows and two more, and an SM's strips share its FP64 pipe: a row takes 0.75
+// us in one or two CTAs of an SM and 0.32 us per CTA beyond, so the height with
+// the least (rows + 2) * max(CTAs per SM, 2.5) is taken.  Once 32 rows leave five
+// CTAs per SM, what registers allow, lower strips only repeat more rows (2050^2:
+// 93 us, 101 with 25 rows).  Strips of 32 rows throughout (6 of them for 64 x 64
+// cells) took 26.6 us per step of every patch up to 700^2; now 9 us at 64^2,
+// 12.6 at 370^2, 16.4 at 500^2, 21.3 at 700^2, 48.6 (52.0) at 1400^2.
+static int fv_strip_rows(long nx, long ny) {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const long cols = (nx + FVS_WARPS * FVS_W - 1) / (FVS_WARPS * FVS_W);
+  int best = FVS_H;
+  long least = -1;
+  for (int h = FVS_H; h >= 1; h--) {
+    const long ctas = (cols * ((ny + h - 1) / h) + sms - 1) / sms;
+    if (h == FVS_H && ctas > 5) break;
+    const long cost = (h + 2) * (2 * ctas > 5 ? 2 * ctas : 5);
+    if (least < 0 || cost < least) best = h, least = cost;
+  }
+  return best;
+}
+
 template <bool PLANAR, bool GRID>
 __global__ void __launch_bounds__(32 * FVS_WARPS) k_fv_godunov_sweep(FVArgs a) {
   constexpr int V = kV, C = kV + 1;
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
   const int NX = GRID ? a.P * a.npx : a.P, NY = GRID ? a.P * a.npy : a.P;
   const int c = (blockIdx.x * FVS_WARPS + w) * FVS_W - 1 + l;  // this lane's column
-  const int j0 = blockIdx.y * FVS_H;
+  const int H = a.rows, j0 = blockIdx.y * H;
   const bool out_col = l >= 1 && l <= FVS_W && c < NX;
   const double dtv = *a.dt_dev;
   const double cx = dtv / a.hx, cy = dtv / a.hy;
@@ -249,13 +295,13 @@ __global__ void __launch_bounds__(32 * FVS_WARPS) k_fv_godunov_sweep(FVArgs a) {
   for (int m = 0; m < V; m++) part[m] = 0.0;
   double un[V];
   load(j0, un, &rc_n);
-  for (int i = 0; i <= FVS_H; i++) {
+  for (int i = 0; i <= H; i++) {
     const int r = j0 + i;
     double u[V];
 #pragma unroll
     for (int m = 0; m < V; m++) u[m] = un[m];
     rc_u = rc_n;
-    if (i < FVS_H) load(r + 1, un, &rc_n);  // prefetch the next row
+    if (i < H) load(r + 1, un, &rc_n);  // prefetch the next row
     double cyr[C];
     fv_cell_flux<PLANAR>(u, 1, cyr);
     // the face below row r: bottom face of row r, top face of row r - 1
@@ -273,7 +319,7 @@ __global__ void __launch_bounds__(32 * FVS_WARPS) k_fv_godunov_sweep(FVArgs a) {
       for (int m = 0; m < V; m++) o[m] = v[m];
       ndt.add<PLANAR>(v);
     }
-    if (i == FVS_H) break;
+    if (i == H) break;
     // x faces of row r: the left one from this lane and its left neighbour,
     // the right one from the right neighbour lane
     double cxr[C];
@@ -1263,8 +1309,9 @@ exa_status_t fv_patch_step_async(int scheme, const exa_fv_desc_t& d, const doubl
       gattr[planar] = true;
     }
     if (tune_get(kTuneFvGodunov, 0) != 1) {
+      a.rows = fv_strip_rows(d.patch, d.patch);
       const dim3 gs((unsigned)((d.patch + FVS_WARPS * FVS_W - 1) / (FVS_WARPS * FVS_W)),
-                    (unsigned)((d.patch + FVS_H - 1) / FVS_H), 1);
+                    (unsigned)((d.patch + a.rows - 1) / a.rows), 1);
       if (planar) k_fv_godunov_sweep<true, false><<<gs, 32 * FVS_WARPS, 0, st>>>(a);
       else k_fv_godunov_sweep<false, false><<<gs, 32 * FVS_WARPS, 0, st>>>(a);
     } else if (planar) {
@@ -1989,8 +2036,9 @@ static exa_status_t fv_patchgrid_step_one(exa_fv_patchgrid* g) {
       gattr[planar] = true;
     }
     if (tune_get(kTuneFvGodunov, 0) != 1) {
+      a.rows = fv_strip_rows(NX, NY);
       const dim3 gs((unsigned)((NX + FVS_WARPS * FVS_W - 1) / (FVS_WARPS * FVS_W)),
-                    (unsigned)((NY + FVS_H - 1) / FVS_H), 1);
+                    (unsigned)((NY + a.rows - 1) / a.rows), 1);
       if (planar) k_fv_godunov_sweep<true, true><<<gs, 32 * FVS_WARPS, 0, g->st>>>(a);
       else k_fv_godunov_sweep<false, true><<<gs, 32 * FVS_WARPS, 0, g->st>>>(a);
     } else {
