@@ -168,12 +168,25 @@ static exa_status_t launch_dn(const exa_aderdg_desc_t& d, const PredArgs& a, int
   // (156,000 to 27,641 cells), 3D orders 3..5 1780 / 2253, 3333 / 4073,
   // 2365 / 2823 (82,000, 68,921 and 15,000 cells).  In 3D order 2 (27 threads
   // a cell, 45 T tasks on them) it measured 1794 against 1757 for line-owner.
+  // Few 2D cells of orders 2 and 5: the line-owner form while one wave of it
+  // holds them.  It spreads a cell's work over more threads, whose chain is all
+  // that counts there: order 5 18.4 / 24.6 us at 24 cells, 20.7 / 24.6 at 576,
+  // but 38.9 / 27.0 at 625 (four CTAs of a cell per SM); order 2 10.2 / 11.3 us
+  // at 400 to 1156 cells, level at 2025.
   // knob 3 selects another: 1 = node-gather, 2 = line-owner contraction, 3 =
-  // the progressive line-owner form (order 4; others line-owner).  Node-gather
-  // also serves the reference-temporaries mode and parameters.
+  // the progressive line-owner form (order 4; others line-owner), 4 = pencil for
+  // any number of cells.  Node-gather also serves the reference-temporaries mode
+  // and parameters.
   const int variant = tune_get(kTuneFp64Variant, 0);
+  bool few = false;
+  if (DIM == 2 && (N == 2 || N == 5) && variant == 0) {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    few = a.ncells <= (N == 2 ? 8L : 4L) * sms;
+  }
   if constexpr (!(DIM == 3 && N == 2))
-    if (d.npar == 0 && !full && variant == 0) {
+    if (d.npar == 0 && !full && (variant == 0 || variant == 4) && !few) {
       if constexpr (DIM == 2)
         if (planar) return launch_pencil<DIM, N, true>(a, st);
       if (planar) return set_error(EXA_EINVAL, "planar Euler is a 2D PDE");

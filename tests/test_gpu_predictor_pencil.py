@@ -87,3 +87,29 @@ def test_cells_of_nan(dim, order, cells):
         else:
             assert ia[c] == ig[c]
             assert all(np.array_equal(a[n][c], good[n][c]) for n in a)
+
+
+@pytest.mark.parametrize('order,cells', [(2, 1), (2, 29), (2, 1184), (2, 1185), (5, 1), (5, 11), (5, 592), (5, 593)])
+def test_few_2d_cells(order, cells):
+    """Orders 2 and 5 take the line-owner form for few 2D cells (8 and 4 per SM;
+    the sizes are those of 148 SMs): default, pencil (key 3 = 4) and line-owner
+    (key 3 = 2) agree to the roundings above, with NaN cells among the others."""
+    rng = np.random.default_rng(cells + order)
+    nn = (order + 1) ** 2
+    q = np.zeros((cells, nn, V))
+    q[..., 0] = 1.0 + 0.1 * rng.random((cells, nn))
+    q[..., 1:4] = 0.1 * rng.standard_normal((cells, nn, 3))
+    q[..., 4] = 2.5 + 0.1 * rng.random((cells, nn))
+    if cells > 10:
+        q[3] = np.nan
+        q[7, nn // 2, 1] = np.nan
+    dx, dt = [0.05, 0.04], 3e-4
+    a, ia = run(0, 2, order, cells, q, dx, dt, E.PDE_EULER)
+    for variant in (2, 4):
+        b, ib = run(variant, 2, order, cells, q, dx, dt, E.PDE_EULER)
+        assert np.array_equal(ia, ib)
+        for n in a:
+            assert np.array_equal(np.isnan(a[n]), np.isnan(b[n]))
+            # lduh is a difference of fluxes (about 3) over dx
+            scale = 3.0 / min(dx) if n == 'lduh' else np.nanmax(np.abs(a[n]))
+            assert np.nanmax(np.abs(a[n] - b[n])) <= (1e-12 if n == 'lduh' else 1e-13) * scale
