@@ -163,9 +163,7 @@ def measured_peaks():
 def fp64_predictor_kernel(order):
     """The FP64 predictor kernel the library launches for 3D Euler at this
     order by default (tuning key 3 unset)."""
-    if order == 4:
-        return 'k_predictor_prog'
-    return 'k_predictor_lines' if order >= 4 else 'k_predictor'
+    return 'k_predictor_lines' if order == 2 else 'k_predictor_pencil'
 
 
 def mixed_predictor_kernel(order, variant=0):

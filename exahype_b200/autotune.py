@@ -28,9 +28,9 @@ def _time_ensemble(ens, steps):
 
 def tune_contraction(ens, steps=3, mask=0x30):
     """Coordinate descent over the contraction of each order present
-    (line-owner or node-gather; exa_ensemble_tune_contraction) in the
-    ensemble's current launch form and schedule, from `mask` (default: the
-    library's, orders 4 and 5 line-owner), flipping one order at a time and
+    (pencil or line-owner against node-gather; exa_ensemble_tune_contraction)
+    in the ensemble's current launch form and schedule, from `mask` (the
+    library's defaults: 0x3c in FP64, 0x30 mixed), flipping one order at a time and
     keeping the faster.  Applies the result and returns (mask, table)."""
     table = []
     present = sorted({c.order for c in ens.cfgs.values()})
@@ -55,8 +55,8 @@ def tune_ensemble(ens, steps=3, ctas=(1, 2), grabs=(1, 2, 4, 8), orders=(0, 1), 
     """Picks the ensemble's knobs by timing `ens` itself (which advances
     while being measured):
 
-    1. the contraction of each order present (line-owner or node-gather;
-       exa_ensemble_tune_contraction): coordinate descent from the default,
+    1. the contraction of each order present (pencil or line-owner against
+       node-gather; exa_ensemble_tune_contraction): coordinate descent,
        flipping one order at a time and keeping the faster;
     2. the persistent schedule: CTAs per SM x work items per atomic grab
        (the cells-per-CTA schedule: a grab takes that many consecutive
@@ -78,7 +78,7 @@ def tune_ensemble(ens, steps=3, ctas=(1, 2), grabs=(1, 2, 4, 8), orders=(0, 1), 
             ens.set_launch_mode(lm)
             return tuple(got['best']), got['table']
     table = []
-    mask = 0x30  # orders 4 and 5 line-owner: the library's default
+    mask = 0x30  # start of the descent: orders 4 and 5
     if contraction and ens.cfgs:
         ens.tune(ctas[0], grabs[0], orders[0])
         mask, table = tune_contraction(ens, steps, mask)

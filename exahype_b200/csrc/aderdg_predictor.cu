@@ -164,9 +164,9 @@ static exa_status_t launch_dn(const exa_aderdg_desc_t& d, const PredArgs& a, int
   const bool planar = d.pde == EXA_PDE_EULER_PLANAR;
   // Default: the pencil form, except 3D order 2.  us per call, pencil against
   // the faster of the other forms (node-gather, line-owner, progressive
-  // line-owner): 2D orders 2..5 308 / 478, 396 / 524, 541 / 721, 566 / 845
-  // (156,000 to 27,641 cells), 3D orders 3..5 1780 / 2253, 3333 / 4073,
-  // 2365 / 2823 (82,000, 68,921 and 15,000 cells).  In 3D order 2 (27 threads
+  // line-owner): 2D orders 2..5 309 / 478, 398 / 524, 544 / 721, 578 / 845
+  // (156,000 to 27,641 cells), 3D orders 3..5 1648 / 2253, 3337 / 4073,
+  // 2371 / 2823 (82,000, 68,921 and 15,000 cells).  In 3D order 2 (27 threads
   // a cell, 45 T tasks on them) it measured 1794 against 1757 for line-owner.
   // Few 2D cells of orders 2 and 5: the line-owner form while one wave of it
   // holds them.  It spreads a cell's work over more threads, whose chain is all

@@ -19,7 +19,8 @@
 // 10 (3D) or 6 (2D) doubles and three or two barriers per iteration, every
 // thread has B independent fluxes (their divisions overlap), and cells are
 // packed without padding to a power of two or to whole warps (2D order 5:
-// three cells of 36 threads in 128 instead of two; order 2: 14 instead of 8).
+// five cells of 36 threads in 192 instead of three; order 2: 14 in 128 instead
+// of 8).
 //
 // The arrays [n][z][y][x][variable] are padded so that every access above is
 // free of bank conflicts or nearly so (16 banks of 8 bytes per half-warp).

@@ -359,8 +359,8 @@ __global__ void __launch_bounds__(32 * FVS_WARPS) k_fv_godunov_sweep(FVArgs a) {
 // single patches leaves most of a tile empty here (10 x 10 patches fill 100
 // of 2 x 256 cells) and re-reads the ghost rows per tile: 40,000 patches of
 // 10 x 10 took it 1259 us and the call 1.29 ms (with a host-made +inf array and
-// a synchronisation for the admissible dt); this way the call takes 0.17 ms,
-// bound by HBM (620 MB: luh once, luh_new in and out).
+// a synchronisation for the admissible dt); this way the kernel takes 0.18 ms,
+// bound by memory latency (640 MB: luh once, luh_new in and out).
 // As in the reference, the update is applied to luh_new as it is, and the
 // faces of the patch boundary also reach its first ghost layer: a ghost
 // column belongs to its lane, a ghost row to the lanes above or below it.

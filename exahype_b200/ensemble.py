@@ -67,7 +67,8 @@ class Ensemble:
         call('exa_ensemble_tune', self.h, int(ctas_per_sm), int(grab), int(order_policy))
 
     def tune_contraction(self, lines_mask):
-        """Per order N: bit N set = line-owner contraction, clear = node-gather."""
+        """Per order N: bit N set = pencil (FP64) or line-owner (mixed)
+        contraction, clear = node-gather."""
         call('exa_ensemble_tune_contraction', self.h, int(lines_mask))
 
     def set_launch_mode(self, mode):

@@ -115,8 +115,10 @@ exa_status_t exa_dropin_workspace_doubles(int device, size_t* doubles);
  * 2D order 5); 0: progressive for 3D order 4 Euler and 2D order 5,
  * line-owner for the other orders >= 4, node-gather otherwise), 3 = the same
  * for the FP64 predictor (1: node-gather, 2: line-owner, 3: progressive
- * line-owner, order 4 (3D: Euler); 0: progressive for order 4 (3D: Euler),
- * line-owner for the other orders >= 4, node-gather otherwise), 4 = cells per CTA of the limiter kernels (0: automatic),
+ * line-owner, order 4 (3D: Euler), line-owner for other orders, 4: space-time
+ * pencil, line-owner for 3D order 2; 0: pencil, but line-owner for 3D order 2 and
+ * for few 2D cells of orders 2 and 5), 4 = cells per CTA of the limiter kernels
+ * (0: automatic),
  * 5 = the fused 2D Godunov step (one patch, the patch grid; 1: 32 x 8 tile
  * kernel; otherwise the sweep kernel, warps walking up strips of rows).  exa_tune_get
  * returns -1 for keys never set. */
@@ -601,8 +603,9 @@ exa_status_t exa_ensemble_use_graph(exa_ensemble* e, int enable);
  * atomic grab, work order (0 = costly orders first, 1 = solve order) */
 exa_status_t exa_ensemble_tune(exa_ensemble* e, int ctas_per_sm, int grab, int order_policy);
 /* contraction of each order's predictor inside the persistent launch: bit N
- * of lines_mask set = line-owner contraction, clear = node-gather (default:
- * orders 4 and 5 line-owner); results agree to rounding */
+ * of lines_mask set = pencil (FP64) or line-owner (mixed) contraction, clear =
+ * node-gather (default: every order in FP64, orders 4 and 5 in mixed); results
+ * agree to rounding */
 exa_status_t exa_ensemble_tune_contraction(exa_ensemble* e, int lines_mask);
 /* launch form of a step: 0 (default) one persistent cooperative launch
  * (work items taken from an atomic counter, grid barriers between the
