@@ -372,13 +372,28 @@ struct FVStrips {
   int rows;      // rows of a block
 };
 
-__host__ __device__ inline FVStrips fv_strips(int P, long npatches) {
+static FVStrips fv_strips(int P, long npatches) {
   FVStrips s;
   s.width = P < 30 ? P : 30;
   s.per_warp = 32 / (s.width + 2);
   s.across = (P + s.width - 1) / s.width;
-  // whole columns up to 32 rows, blocks of 32 above (two halo rows each)
+  // whole columns up to 32 rows, blocks of 32 above (two halo rows each); fewer
+  // rows for few patches, as in fv_strip_rows (patches side by side in a warp
+  // keep whole columns: a warp's strips have one length): 50 patches of 15 x 15
+  // 20 -> 12.9 us per call, of 32 x 32 37.8 -> 16.2, of 64 x 64 37.6 -> 20.8
   s.rows = P <= 32 ? P : 32;
+  if (s.per_warp == 1) {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    long least = -1;
+    for (int h = s.rows, top = s.rows; h >= 1; h--) {
+      const long ctas = ((npatches * s.across * ((P + h - 1) / h) + FVS_WARPS - 1) / FVS_WARPS + sms - 1) / sms;
+      if (h == top && ctas > 4) break;
+      const long cost = (h + 2) * (2 * ctas > 5 ? 2 * ctas : 5);
+      if (least < 0 || cost < least) s.rows = h, least = cost;
+    }
+  }
   s.up = (P + s.rows - 1) / s.rows;
   s.units = npatches * s.across * s.up;
   return s;
@@ -391,10 +406,11 @@ __global__ void __launch_bounds__(32 * FVS_WARPS) k_fv_godunov_batch(FVArgs a, F
   const int LP = st.width + 2;
   const int sub = l / LP, c = l - sub * LP;
   const long warp = (long)blockIdx.x * FVS_WARPS + (threadIdx.x >> 5);
-  const long unit = warp * st.per_warp + sub;
-  const bool live = sub < st.per_warp && unit < st.units;
-  const long patch = live ? unit / (st.across * st.up) : 0;
-  const int part_i = live ? (int)(unit - patch * (st.across * st.up)) : 0;
+  // (lanes beyond the last strip walk along with it)
+  const long unit = warp * st.per_warp + (sub < st.per_warp ? sub : st.per_warp - 1);
+  const bool have = unit < st.units, live = sub < st.per_warp && have;
+  const long patch = have ? unit / (st.across * st.up) : 0;
+  const int part_i = have ? (int)(unit - patch * (st.across * st.up)) : 0;
   const int sx = part_i % st.across, sy = part_i / st.across;
   const int S = a.S, D = kV + a.npar, pb = a.g, pe = a.g + a.P;
   const int k = pb - 1 + sx * st.width + c;
