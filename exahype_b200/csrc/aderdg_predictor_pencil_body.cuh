@@ -82,7 +82,9 @@ __device__ const unsigned char kPencilY34[125] = {
     121, 106, 107, 108, 97,  98,  99,  112, 113, 114, 116, 117, 119, 120, 122, 123, 124, 109, 110, 111};
 
 // Sum of v over the threads of each cell (every thread of the CTA calls it;
-// threads outside a cell pass cell -1).  One barrier; the partials go to one
+// threads outside a cell pass cell -1).  The order depends on where the cell
+// lies in the CTA; the parts are multiples of 2^-98 (kPicardBase), so the sum
+// does not where it matters.  One barrier; the partials go to one
 // of two sets chosen by the iteration's parity, so the next call's stores
 // never meet this call's loads.
 template <typename S>
@@ -264,16 +266,19 @@ __device__ __forceinline__ void predictor_pencil_block(const PredArgs& a, long b
   for (int iter = 0;; iter++) {
     // the new pencil and its squared increment
     double qn[B][V], r2 = 0.0;
-    if (valid && !done)
+    if (valid && !done) {
+      r2 = kPicardBase;
 #pragma unroll
       for (int x = 0; x < B; x++)
 #pragma unroll
         for (int m = 0; m < V; m++) {
           const double v = sG[own + x * V + m];
           const double d = q[x][m] - v;
-          r2 += d * d;
+          r2 = fma(d, d, r2);
           if (kHold) qn[x][m] = v;
         }
+      r2 -= kPicardBase;
+    }
     if (lost && valid && !done) {
       bool all = true;
 #pragma unroll
@@ -285,7 +290,7 @@ __device__ __forceinline__ void predictor_pencil_block(const PredArgs& a, long b
     const double res = pencil_sum<S>(r2, lc, s, sred, iter);
     if (!done) {
       it = res == TPC * kVote ? MAXIT : iter + 1;
-      conv = res >= 0.0 && res < 1e-7 * 1e-7;
+      conv = res >= 0.0 && res < kPicardTol2;
       lost = !(res >= 0.0);
       done = conv || it == MAXIT;
       // the outputs need the last iteration's input (for its flux), put in

@@ -99,6 +99,18 @@ __device__ __forceinline__ void cp_async_commit_wait_all() {
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
 }
 
+// ------------------------------------------- residual of the Picard loop
+// Sum of squared increments that does not depend on the order of its terms
+// when it is compared with the tolerance.  An accumulator starts at 2^-46, so
+// that every square is rounded to a multiple of 2^-98 as it is added (a square
+// is never half way between two of them: its lowest bit has an even exponent).
+// Below 2^-45 such sums are exact, and one that leaves this range is above the
+// tolerance whatever its rounding.  Which lanes and warps add up a cell, and
+// in which order, therefore never decides when its iteration stops.
+constexpr double kPicardBase = 0x1p-46;
+constexpr double kPicardTol2 = 1e-7 * 1e-7;
+static_assert(kPicardTol2 < kPicardBase, "the tolerance lies in the exact range");
+
 // ------------------------------------------------------------ reductions
 // Sum over groups of G consecutive threads (G a power of two <= 32, or a
 // multiple of 32).  Every thread of a group returns the bitwise identical
