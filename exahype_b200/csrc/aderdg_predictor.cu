@@ -173,6 +173,8 @@ static exa_status_t launch_dn(const exa_aderdg_desc_t& d, const PredArgs& a, int
   // that counts there: order 5 18.4 / 24.6 us at 24 cells, 20.7 / 24.6 at 576,
   // but 38.9 / 27.0 at 625 (four CTAs of a cell per SM); order 2 10.2 / 11.3 us
   // at 400 to 1156 cells, level at 2025.
+  // Both forms give a cell the same bits, so that neither the cells beside it in
+  // a call nor the cut of a grid into slabs shows in its values.
   // knob 3 selects another: 1 = node-gather, 2 = line-owner contraction, 3 =
   // the progressive line-owner form (order 4; others line-owner), 4 = pencil for
   // any number of cells.  Node-gather also serves the reference-temporaries mode

@@ -56,6 +56,10 @@ __device__ __forceinline__ void predictor_fp64_lines_block(const PredArgs& a, lo
   using S = Fp64LineShape<DIM, N>;
   constexpr int B = S::B, V = S::V, NPC = S::NPC, G = S::G, L = S::L, TPD = S::TPD, TPT = S::TPT;
   constexpr int MAXIT = 2 * (N + 1);
+  // 2D orders 2 and 5 share their calls with the pencil form (few cells run
+  // here, many there), so a cell's values must be the same in both: the same
+  // operations in the same order
+  constexpr bool kAsPencil = DIM == 2 && (N == 2 || N == 5);
   const DGConst& T = c_dg[N];
 
   const int lc = threadIdx.x / G;
@@ -189,19 +193,25 @@ __device__ __forceinline__ void predictor_fp64_lines_block(const PredArgs& a, lo
           const int ns = iter == 0 ? 0 : n;
           double g = 0.0;
 #pragma unroll
-          for (int d = 0; d < DIM; d++) g += a.idx[d] * sX[((d * B + ns) * V + m) * NPC + s];
+          for (int d = 0; d < DIM; d++) g = fma(a.idx[d], sX[((d * B + ns) * V + m) * NPC + s], g);
 #pragma unroll
-          for (int t = 0; t < B; t++) acc[t][m] += T.tA[t][n] * g;
+          for (int t = 0; t < B; t++) {
+            // (slices that all hold the same value: the sum of their weights)
+            if (kAsPencil && iter == 0) acc[t][m] = n == 0 ? T.tAsum[t] * g : acc[t][m];
+            else acc[t][m] = fma(T.tA[t][n], g, acc[t][m]);
+          }
         }
+      r2 = kPicardBase;
 #pragma unroll
       for (int t = 0; t < B; t++)
 #pragma unroll
         for (int m = 0; m < V; m++) {
-          const double qn = T.c0[t] * lu[m] - dt * acc[t][m];
+          const double qn = picard_new(T.c0[t], lu[m], dt, acc[t][m]);
           const double dq = q[t][m] - qn;
-          r2 += dq * dq;
+          r2 = fma(dq, dq, r2);
           q[t][m] = qn;
         }
+      r2 -= kPicardBase;
       if (kShared)
 #pragma unroll
         for (int d = 0; d < DIM; d++)
@@ -213,7 +223,7 @@ __device__ __forceinline__ void predictor_fp64_lines_block(const PredArgs& a, lo
     const double res = group_sum_1b<G, S::NT>(r2, sred, iter);
     if (!conv) {
       it = iter + 1;
-      if (res < 1e-7 * 1e-7) conv = true;
+      if (res < kPicardTol2) conv = true;
     }
     if constexpr (S::CPB == 1) {
       if (conv || !valid) break;

@@ -129,7 +129,7 @@ __device__ __forceinline__ void predictor_fp64_prog_block(const PredArgs& a, lon
       for (int m = 0; m < V; m++) {
         double g = 0.0;
 #pragma unroll
-        for (int d = 0; d < DIM; d++) g += a.idx[d] * X[(d * V + m) * NPC + s];
+        for (int d = 0; d < DIM; d++) g = fma(a.idx[d], X[(d * V + m) * NPC + s], g);
         if (iter == 0) {
 #pragma unroll
           for (int n2 = 0; n2 < B; n2++)
@@ -192,22 +192,24 @@ __device__ __forceinline__ void predictor_fp64_prog_block(const PredArgs& a, lon
     // new iterate into acc (the old one stays in q until the exit test)
     double r2 = 0.0;
     if (active && !conv) {
+      r2 = kPicardBase;
 #pragma unroll
       for (int t = 0; t < B; t++)
 #pragma unroll
         for (int m = 0; m < V; m++) {
           // luh re-read (read-only path, L1): ten fewer registers across
           // the slice loop
-          const double qn = T.c0[t] * __ldg(a.luh + cell * (long)NPC * V + s * V + m) - dt * acc[t][m];
+          const double qn = picard_new(T.c0[t], __ldg(a.luh + cell * (long)NPC * V + s * V + m), dt, acc[t][m]);
           const double dq = q[t][m] - qn;
-          r2 += dq * dq;
+          r2 = fma(dq, dq, r2);
           acc[t][m] = qn;
         }
+      r2 -= kPicardBase;
     }
     const double res = group_sum_1b<G, S::NT>(r2, sred, iter);
     if (!conv) {
       it = iter + 1;
-      if (res < 1e-7 * 1e-7) conv = true;
+      if (res < kPicardTol2) conv = true;
     }
     const bool last = conv || iter == MAXIT - 1;
     if (last && active && (!kMulti || !done)) {

@@ -234,13 +234,13 @@ __device__ __forceinline__ void predictor_pencil_block(const PredArgs& a, long b
           double d = 0.0;
 #pragma unroll
           for (int p = 0; p < B; p++) d += T.deriv[i][p] * f[p];
-          g[i] += a.idx[DIM - 1] * d;
+          g[i] = fma(a.idx[DIM - 1], d, g[i]);
         }
 #pragma unroll
         for (int i = 0; i < B; i++) {
           const double u = luh[i * TG + k];
 #pragma unroll
-          for (int t = 0; t < B; t++) sG[o + t * SLICE + i * TS] = T.c0[t] * u - dt * (T.tAsum[t] * g[i]);
+          for (int t = 0; t < B; t++) sG[o + t * SLICE + i * TS] = picard_new(T.c0[t], u, dt, T.tAsum[t] * g[i]);
         }
       }
     }
@@ -396,16 +396,16 @@ __device__ __forceinline__ void predictor_pencil_block(const PredArgs& a, long b
             double d = 0.0;
 #pragma unroll
             for (int p = 0; p < B; p++) d += T.deriv[i][p] * f[p];
-            const double g = sG[o + n * SLICE + i * TS] + a.idx[DIM - 1] * d;
+            const double g = fma(a.idx[DIM - 1], d, sG[o + n * SLICE + i * TS]);
 #pragma unroll
-            for (int t = 0; t < B; t++) acc[t][i] += T.tA[t][n] * g;
+            for (int t = 0; t < B; t++) acc[t][i] = fma(T.tA[t][n], g, acc[t][i]);
           }
         }
 #pragma unroll
         for (int i = 0; i < B; i++) {
           const double u = __ldg(luh + i * TG + k);
 #pragma unroll
-          for (int t = 0; t < B; t++) sG[o + t * SLICE + i * TS] = T.c0[t] * u - dt * acc[t][i];
+          for (int t = 0; t < B; t++) sG[o + t * SLICE + i * TS] = picard_new(T.c0[t], u, dt, acc[t][i]);
         }
       }
     __syncthreads();

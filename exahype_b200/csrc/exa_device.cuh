@@ -110,6 +110,11 @@ __device__ __forceinline__ void cp_async_commit_wait_all() {
 constexpr double kPicardBase = 0x1p-46;
 constexpr double kPicardTol2 = 1e-7 * 1e-7;
 static_assert(kPicardTol2 < kPicardBase, "the tolerance lies in the exact range");
+// a new iterate, c0 u - dt sum: the difference of two products can be fused
+// either way round, and kernels that share a cell's calls must agree on it
+__device__ __forceinline__ double picard_new(double c0, double u, double dt, double sum) {
+  return fma(c0, u, -(dt * sum));
+}
 
 // ------------------------------------------------------------ reductions
 // Sum over groups of G consecutive threads (G a power of two <= 32, or a
