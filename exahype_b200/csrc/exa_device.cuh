@@ -192,6 +192,16 @@ __device__ __forceinline__ void atomic_min_pos_double(unsigned long long* addr, 
   if (v >= 0.0) atomicMin(addr, (unsigned long long)__double_as_longlong(v));
 }
 
+// Dynamic shared memory that kernels of call-dependent size may be launched
+// with.  The limit belongs to the function, not to the launch: it is always set
+// to this value, for a call that set its own smaller need could make the launch
+// of another thread, between that thread's setting and its launch, fail.
+constexpr size_t kMaxDynSmem = 200 * 1024;
+template <class K>
+inline cudaError_t allow_max_smem(K kern) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem);
+}
+
 constexpr int next_pow2(int x) { int p = 1; while (p < x) p <<= 1; return p; }
 constexpr int round_up(int x, int m) { return (x + m - 1) / m * m; }
 constexpr int ipow(int b, int e) { return e == 0 ? 1 : b * ipow(b, e - 1); }

@@ -1432,8 +1432,8 @@ static exa_status_t fv_update(int scheme, const exa_fv_desc_t* desc, long npatch
   if (desc->patch <= kFvSmallMax) {
     auto kern = planar ? k_fv_patch_small<true, 1, true> : k_fv_patch_small<false, 1, true>;
     const size_t smem = fv_small_smem(desc->patch, desc->ghost, 1);
-    if (smem <= 200 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem <= kMaxDynSmem) {
+      cudaError_t e = allow_max_smem(kern);
       if (e != cudaSuccess) return cuda_status(e, "muscl batch attribute");
       kern<<<(unsigned)npatches, FVS_NT, smem, st>>>(a);
       count_launch();
@@ -1971,7 +1971,7 @@ exa_status_t fv_subcell_step(int scheme, int planar, int P, int g, int npx, int 
   const size_t smem = fv_small_smem(P, g, scheme);
   auto kern = scheme == 0 ? (planar ? k_fv_patch_small<true, 0, false> : k_fv_patch_small<false, 0, false>)
                           : (planar ? k_fv_patch_small<true, 1, false> : k_fv_patch_small<false, 1, false>);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_max_smem(kern);
   if (e != cudaSuccess) return cuda_status(e, "subcell FV attribute");
   const long grid = maxcells < 16L * sms ? maxcells : 16L * sms;  // CTAs loop over the listed patches
   kern<<<(unsigned)grid, FVS_NT, smem, st>>>(a);

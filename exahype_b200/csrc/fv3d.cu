@@ -245,7 +245,7 @@ exa_status_t fv3_update(int scheme, int P, int g, int D, const double* h, long n
                         const double* luh, double dt, const double* dt_dev, double* max_dt, const int* list,
                         const int* count, cudaStream_t st) {
   const size_t smem = fv3_smem(P, g, scheme);
-  if (smem > 200 * 1024) return set_error(EXA_EINVAL, "3D FV: patch too large for one CTA");
+  if (smem > kMaxDynSmem) return set_error(EXA_EINVAL, "3D FV: patch too large for one CTA");
   FV3Args a{};
   a.P = P;
   a.g = g;
@@ -260,7 +260,7 @@ exa_status_t fv3_update(int scheme, int P, int g, int D, const double* h, long n
   a.list = list;
   a.count = count;
   auto kern = scheme == 0 ? k_fv3_patch<0> : k_fv3_patch<1>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_max_smem(kern);
   if (e != cudaSuccess) return cuda_status(e, "3D FV attribute");
   long grid = npatches;
   if (count) {

@@ -39,7 +39,7 @@ constexpr int kLimMaxOrder = 6;  // B <= 7, S <= 13
 constexpr int kLimNT = 256;
 constexpr int kLimColNT = 128;  // threads of the projections
 constexpr int kLimMmNT = 128;   // and of the extrema
-constexpr int kLimMaxSmem = 200 * 1024;
+constexpr int kLimMaxSmem = (int)kMaxDynSmem;
 
 struct LimConst {
   double uh2lim[7][13];  // [k][i]: mean of phi_k over subcell i
@@ -623,11 +623,6 @@ static int lim_cpb(long items_per_cell, long smem_per_cell, long ncells, int nt,
   return best;
 }
 
-template <class K>
-static cudaError_t lim_prepare(K kern, size_t smem) {
-  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-}
-
 template <int DIM, int B, int NVT>
 static exa_status_t lim_run(int op, int nvar, int nobs, int ghost, long ncells, const double* in, double* out,
                             double* mn, double* mx, int* ok, double relax, double scaling, cudaStream_t st,
@@ -685,7 +680,7 @@ static exa_status_t lim_run(int op, int nvar, int nobs, int ghost, long ncells, 
         // shared memory (order 4: 6,000 cells; beyond, the streamed planes are
         // level or better)
         if (!cpb_set && !sel.list && few <= kLimMaxSmem && ncells * few <= 10L * sms * kLimMaxSmem) {
-          cudaError_t e = lim_prepare(k_lim_to_dg_few<B, NVT>, (size_t)few);
+          cudaError_t e = allow_max_smem(k_lim_to_dg_few<B, NVT>);
           if (e != cudaSuccess) return cuda_status(e, "limiter: shared-memory attribute");
           k_lim_to_dg_few<B, NVT><<<(unsigned)ncells, kLimNT, (size_t)few, st>>>(nvar, ghost, ncells, in, out);
           count_launch();
@@ -699,7 +694,7 @@ static exa_status_t lim_run(int op, int nvar, int nobs, int ghost, long ncells, 
     long nblk = (ncells + cpb - 1) / cpb;
     if (sel.count) nblk = nblk < 8L * sms ? nblk : 8L * sms;  // a selection usually holds a few cells: CTAs loop
     if (nblk > 0x7fffffffL) return set_error(EXA_EINVAL, "limiter: too many cells");
-    cudaError_t e = fv ? lim_prepare(k_lim_to_fv<DIM, B, NVT>, smem) : lim_prepare(k_lim_to_dg<DIM, B, NVT>, smem);
+    cudaError_t e = fv ? allow_max_smem(k_lim_to_fv<DIM, B, NVT>) : allow_max_smem(k_lim_to_dg<DIM, B, NVT>);
     if (e != cudaSuccess) return cuda_status(e, "limiter: shared-memory attribute");
     if (fv)
       k_lim_to_fv<DIM, B, NVT><<<(unsigned)nblk, nt, smem, st>>>(nvar, ghost, ncells, cpb, in, out, sel);
@@ -732,7 +727,7 @@ static exa_status_t lim_run(int op, int nvar, int nobs, int ghost, long ncells, 
   if (nblk > 0x7fffffffL) return set_error(EXA_EINVAL, "limiter: too many cells");
   cudaError_t e = cudaSuccess;
   if (op == kLimFvMinMax) {
-    e = lim_prepare(k_lim_fv_min_max<DIM, B>, smem);
+    e = allow_max_smem(k_lim_fv_min_max<DIM, B>);
     if (e == cudaSuccess)
       k_lim_fv_min_max<DIM, B><<<(unsigned)nblk, kLimNT, smem, st>>>(nvar, nobs, ghost, ncells, cpb, in, mn, mx,
                                                                        sel);
@@ -740,7 +735,7 @@ static exa_status_t lim_run(int op, int nvar, int nobs, int ghost, long ncells, 
     auto kern = k_lim_min_max<DIM, B, NVT, false>;
     if constexpr (DIM == 2 && B <= 6)
       if (walk) kern = k_lim_min_max<DIM, B, NVT, true>;
-    e = lim_prepare(kern, smem);
+    e = allow_max_smem(kern);
     if (e == cudaSuccess)
       kern<<<(unsigned)nblk, kLimMmNT, smem, st>>>(op == kLimDmp ? 1 : 0, nvar, nobs, ncells, cpb, in, relax, scaling, mn,
                                                   mx, ok);
