@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(32 * FVS_WARPS) k_fv_godunov_batch(FVArgs a, F
 // one CTA per small patch (defined with the fused steps below)
 constexpr int FVS_NT = 128;
 constexpr int kFvSmallMax = 16;
-template <bool PLANAR, int SCHEME, bool BATCH>
+template <bool PLANAR, int SCHEME, bool BATCH, int NT = FVS_NT>
 __global__ void k_fv_patch_small(FVArgs a);
 inline size_t fv_small_smem(int P, int g, int scheme) {
   const size_t S = P + 2 * g, R = P + 2;
@@ -1430,12 +1430,29 @@ static exa_status_t fv_update(int scheme, const exa_fv_desc_t* desc, long npatch
   }
   if (exa_status_t s = clear_max_dt()) return s;
   if (desc->patch <= kFvSmallMax) {
-    auto kern = planar ? k_fv_patch_small<true, 1, true> : k_fv_patch_small<false, 1, true>;
+    // Threads per patch: 128, or 256 where a patch of 10 cells or more has an SM
+    // to itself or shares it with one other (50 patches of 12 x 12: 7.0 us, 8.9
+    // with 128; 400: 13.0 against 11.5, since fewer of them are resident), or
+    // 384 for one per SM of 15 and 16 (7.9 us, 9.4 with 256 and 11.7 with 128).
+    // From 15 cells on shared memory leaves two or three CTAs per SM anyhow and
+    // 256 stay ahead (20,000 of 16 x 16: 701 us, 128: 861).  The tile kernel
+    // below, which pads the rows to 32, takes 8.2 us for 50 patches of 10 x 10
+    // (6.6 here), 347 us for 20,000 of 4 x 4 (143), 886 of 10 x 10 (282) and
+    // 1105 of 16 x 16.
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int P = desc->patch;
+    const int nt = P >= 15 && npatches <= sms ? 384 : (P >= 15 || (P >= 10 && npatches <= 2L * sms) ? 256 : 128);
+    auto kern = planar ? (nt == 128 ? k_fv_patch_small<true, 1, true, 128>
+                                    : (nt == 256 ? k_fv_patch_small<true, 1, true, 256> : k_fv_patch_small<true, 1, true, 384>))
+                       : (nt == 128 ? k_fv_patch_small<false, 1, true, 128>
+                                    : (nt == 256 ? k_fv_patch_small<false, 1, true, 256> : k_fv_patch_small<false, 1, true, 384>));
     const size_t smem = fv_small_smem(desc->patch, desc->ghost, 1);
     if (smem <= kMaxDynSmem) {
       cudaError_t e = allow_max_smem(kern);
       if (e != cudaSuccess) return cuda_status(e, "muscl batch attribute");
-      kern<<<(unsigned)npatches, FVS_NT, smem, st>>>(a);
+      kern<<<(unsigned)npatches, nt, smem, st>>>(a);
       count_launch();
       return cuda_status(cudaGetLastError(), "k_fv_patch_small");
     }
@@ -1713,8 +1730,8 @@ __global__ void k_fv_patch_ic(int P, int g, int D, int npx, int npy, double hx, 
 
 namespace exa {
 // Small patches (patch <= 16, the subcell patches of the limiting ADER-DG
-// grid, stepped for a list of troubled cells): one CTA of 128 threads per
-// patch.  The whole patch with its ghosts (contiguous in
+// grid, stepped for a list of troubled cells): one CTA of NT threads (128 for
+// the subcell patches) per patch.  The whole patch with its ghosts (contiguous in
 // memory) is staged in shared memory, MUSCL-Hancock's ring cells compute
 // their evolved face extrapolations, and every interior cell evaluates its
 // own four face fluxes, applies them in the reference's order and writes
@@ -1724,8 +1741,8 @@ namespace exa {
 // BATCH (exa_fv_musclhancock_update): as the reference's per-patch update
 // instead, luh_new += face contributions, also in its first ghost layer, and
 // the admissible dt per patch.
-template <bool PLANAR, int SCHEME, bool BATCH>
-__global__ void __launch_bounds__(FVS_NT) k_fv_patch_small(FVArgs a) {
+template <bool PLANAR, int SCHEME, bool BATCH, int NT>
+__global__ void __launch_bounds__(NT) k_fv_patch_small(FVArgs a) {
   constexpr int V = kV;
   extern __shared__ double sm[];
   const int P = a.P, g = a.g, S = a.S, D = V + a.npar, pb = g, pe = g + P;
@@ -1756,14 +1773,14 @@ __global__ void __launch_bounds__(FVS_NT) k_fv_patch_small(FVArgs a) {
     // divisions (an FP64 division is a long dependent chain)
     const double ihx = 1.0 / hx, ihy = 1.0 / hy;
     if (!BATCH || a.npar == 0) {
-      for (int i = tid; i < S * S * V; i += FVS_NT) su[i] = luh[i];
+      for (int i = tid; i < S * S * V; i += NT) su[i] = luh[i];
     } else {
-      for (int i = tid; i < S * S * V; i += FVS_NT) su[i] = luh[(i / V) * D + i % V];
+      for (int i = tid; i < S * S * V; i += NT) su[i] = luh[(i / V) * D + i % V];
     }
     double dtl = DBL_MAX;  // BATCH: admissible dt over this thread's faces
     __syncthreads();
     if (SCHEME == 1) {
-      for (int i = tid; i < R * R; i += FVS_NT) {
+      for (int i = tid; i < R * R; i += NT) {
         const int j = pb - 1 + i / R, k = pb - 1 + i % R;
         const double* U = &su[(j * S + k) * V];
         const bool has_x = j >= pb && j < pe;
@@ -1823,7 +1840,7 @@ __global__ void __launch_bounds__(FVS_NT) k_fv_patch_small(FVArgs a) {
       }
       __syncthreads();
       // each face's Rusanov flux once (the reference solves every face once)
-      for (int i = tid; i < 2 * P * (P + 1); i += FVS_NT) {
+      for (int i = tid; i < 2 * P * (P + 1); i += NT) {
         if (i < P * (P + 1)) {
           const int r = i / (P + 1), c = i % (P + 1);  // face left of column pb + c, row pb + r
           const int ic = (r + 1) * R + c + 1;
@@ -1840,7 +1857,7 @@ __global__ void __launch_bounds__(FVS_NT) k_fv_patch_small(FVArgs a) {
       __syncthreads();
     } else {
       // per-cell flux and eigenvalue bound, once per cell and direction
-      for (int i = tid; i < 2 * P * R; i += FVS_NT) {
+      for (int i = tid; i < 2 * P * R; i += NT) {
         if (i < P * R) {
           const int j = pb + i / R, k = pb - 1 + i % R;
           fv_cell_flux<PLANAR>(&su[(j * S + k) * V], 0, &scx[i * C]);
@@ -1854,7 +1871,7 @@ __global__ void __launch_bounds__(FVS_NT) k_fv_patch_small(FVArgs a) {
     }
     const double cx = dt / hx, cy = dt / hy;
     double dtn = DBL_MAX;
-    for (int i = tid; i < P * P; i += FVS_NT) {
+    for (int i = tid; i < P * P; i += NT) {
       const int j = pb + i / P, k = pb + i % P;
       const int r = i / P, c = i % P;
       const double* U = &su[(j * S + k) * V];
@@ -1876,19 +1893,31 @@ __global__ void __launch_bounds__(FVS_NT) k_fv_patch_small(FVArgs a) {
         }
       }
       if constexpr (BATCH) {
+        // every value is read before the first is written (one memory latency
+        // instead of one per variable and ghost cell)
         double* o = out + ((long)j * S + k) * D;
+        const bool edge[4] = {c == 0, c == P - 1, r == 0, r == P - 1};
+        const long to[4] = {-(long)D, (long)D, -(long)S * D, (long)S * D};
+        double u[V], ghost[4][V];
+#pragma unroll
+        for (int m = 0; m < V; m++) u[m] = o[m];
+#pragma unroll
+        for (int e4 = 0; e4 < 4; e4++)
+          if (edge[e4])
+#pragma unroll
+            for (int m = 0; m < V; m++) ghost[e4][m] = o[to[e4] + m];
 #pragma unroll
         for (int m = 0; m < V; m++) {
-          double u = o[m];
-          u += cx * fxl[m];
-          u -= cx * fxr[m];
-          u += cy * fyb[m];
-          u -= cy * fyt[m];
-          o[m] = u;
-          if (c == 0) o[m - D] -= cx * fxl[m];
-          if (c == P - 1) o[m + D] += cx * fxr[m];
-          if (r == 0) o[m - (long)S * D] -= cy * fyb[m];
-          if (r == P - 1) o[m + (long)S * D] += cy * fyt[m];
+          double v = u[m];
+          v += cx * fxl[m];
+          v -= cx * fxr[m];
+          v += cy * fyb[m];
+          v -= cy * fyt[m];
+          o[m] = v;
+          if (edge[0]) o[to[0] + m] = ghost[0][m] - cx * fxl[m];
+          if (edge[1]) o[to[1] + m] = ghost[1][m] + cx * fxr[m];
+          if (edge[2]) o[to[2] + m] = ghost[2][m] - cy * fyb[m];
+          if (edge[3]) o[to[3] + m] = ghost[3][m] + cy * fyt[m];
         }
       } else {
         fv_update_store_dt<PLANAR>(a, out + ((long)j * S + k) * D, U, fxl, fxr, fyb, fyt, cx, cy, dtn);
