@@ -378,22 +378,29 @@ static FVStrips fv_strips(int P, long npatches) {
   s.per_warp = 32 / (s.width + 2);
   s.across = (P + s.width - 1) / s.width;
   // whole columns up to 32 rows, blocks of 32 above (two halo rows each); fewer
-  // rows for few patches, as in fv_strip_rows (patches side by side in a warp
-  // keep whole columns: a warp's strips have one length): 50 patches of 15 x 15
-  // 20 -> 12.9 us per call, of 32 x 32 37.8 -> 16.2, of 64 x 64 37.6 -> 20.8
-  s.rows = P <= 32 ? P : 32;
-  if (s.per_warp == 1) {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    long least = -1;
-    for (int h = s.rows, top = s.rows; h >= 1; h--) {
-      const long ctas = ((npatches * s.across * ((P + h - 1) / h) + FVS_WARPS - 1) / FVS_WARPS + sms - 1) / sms;
-      if (h == top && ctas > 4) break;
-      const long cost = (h + 2) * (2 * ctas > 5 ? 2 * ctas : 5);
-      if (least < 0 || cost < least) s.rows = h, least = cost;
+  // rows for few patches, as in fv_strip_rows: 50 patches of 15 x 15 20 -> 12.9 us
+  // per call, of 32 x 32 37.8 -> 16.2, of 64 x 64 37.6 -> 20.8.  A warp's strips
+  // have one length, so patches side by side keep whole columns; where shorter
+  // ones cost less, a warp takes one strip (device time of 50 patches of 10 x 10
+  // 12.9 -> 4.6 us, of 14 x 14 16.5 -> 4.9; the 32 x 8 tiles before the sweep took
+  // 10.1 and 9.8).
+  const int top = P <= 32 ? P : 32;
+  s.rows = top;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  auto ctas = [&](int h, int per_warp) {  // per SM
+    const long warps = (npatches * s.across * ((P + h - 1) / h) + per_warp - 1) / per_warp;
+    return ((warps + FVS_WARPS - 1) / FVS_WARPS + sms - 1) / sms;
+  };
+  auto cost = [](int h, long n) { return (h + 2) * (2 * n > 5 ? 2 * n : 5); };
+  long least = cost(top, ctas(top, s.per_warp));
+  if (ctas(top, s.per_warp) <= 4)
+    for (int h = top - 1; h >= 1; h--) {
+      const long c = cost(h, ctas(h, 1));
+      if (c < least) s.rows = h, least = c;
     }
-  }
+  if (s.rows < top) s.per_warp = 1;
   s.up = (P + s.rows - 1) / s.rows;
   s.units = npatches * s.across * s.up;
   return s;
