@@ -223,7 +223,10 @@ __device__ __forceinline__ void lim_stage_interior(double* A, const double* __re
 // warps per SM.  Per call before -> now: 3D order 4 (24,000 cells) 344 -> 272 us,
 // order 5 (13,888) 817 -> 283, 2D order 3 (375,000) 304 -> 260, order 5
 // (166,666) 798 -> 347.
-template <int DIM, int B, int NVT>
+// FLAT: a plane has fewer values than the CTA has threads, which then share the
+// planes of all cells (40,000 3D cells of order 3 with one variable 62 us, cell
+// by cell 90).
+template <int DIM, int B, int NVT, bool FLAT>
 __global__ void __launch_bounds__(kLimColNT, LimMinB<DIM, B, false>::value)
     k_lim_to_dg(int nvar_rt, int ghost, long ncells, int cpb, const double* __restrict__ lim, double* luh,
                 LimSel sel) {
@@ -239,14 +242,24 @@ __global__ void __launch_bounds__(kLimColNT, LimMinB<DIM, B, false>::value)
     const int nc = (int)min((long)cpb, nce - c0);
     auto stage = [&](int z) {
       double* d = sm + (z & 1) * buf;
-      for (int c = 0; c < nc; c++) {
-        const double* src = lim + sel.cell(c0 + c) * (DIM == 3 ? plane * SG : plane) +
-                            (DIM == 3 ? (z + ghost) * plane : 0) + ghost * row + (long)ghost * nvar;
-        if (kRows) {
-          for (int k = threadIdx.x; k < len; k += kLimColNT)
-            cp_async8(d + c * len + k, src + k + k / (S * nvar) * 2 * ghost * nvar);
-        } else {
-          for (int k = threadIdx.x; k < len; k += kLimColNT) cp_async8(d + c * len + k, src + k);
+      auto cell_plane = [&](int c) {
+        return lim + sel.cell(c0 + c) * (DIM == 3 ? plane * SG : plane) + (DIM == 3 ? (z + ghost) * plane : 0) +
+               ghost * row + (long)ghost * nvar;
+      };
+      if (FLAT) {
+        for (int i = threadIdx.x; i < nc * len; i += kLimColNT) {
+          const int c = i / len, k = i - c * len;
+          cp_async8(d + i, cell_plane(c) + (kRows ? k + k / (S * nvar) * 2 * ghost * nvar : k));
+        }
+      } else {
+        for (int c = 0; c < nc; c++) {
+          const double* src = cell_plane(c);
+          if (kRows) {
+            for (int k = threadIdx.x; k < len; k += kLimColNT)
+              cp_async8(d + c * len + k, src + k + k / (S * nvar) * 2 * ghost * nvar);
+          } else {
+            for (int k = threadIdx.x; k < len; k += kLimColNT) cp_async8(d + c * len + k, src + k);
+          }
         }
       }
       cp_async_commit();
@@ -670,16 +683,29 @@ static exa_status_t lim_run(int op, int nvar, int nobs, int ghost, long ncells, 
         }
       }
     } else {
-      const long spread = ncells / (4 * sms);
+      // a round of columns, but two CTAs for every SM in 3D, four in 2D where
+      // they then hold four cells (with four and single cells, few cells of few
+      // variables waited longer for memory: 3,000 3D cells of order 4, one
+      // variable, 24 us, 38 before; 1,000 2D cells of order 3 3.8 and 4.2)
+      const long two = (ncells + 2 * sms - 1) / (2 * sms);
+      const long spread = DIM == 3 ? two : max(ncells / (4 * sms), min(two, 4L));
       cpb = (int)(kLimColNT / items > 0 ? kLimColNT / items : 1);
-      if (cpb > spread) cpb = (int)(spread > 0 ? spread : 1);
+      if (cpb > spread) cpb = (int)spread;
       while (cpb > 1 && cpb * per_cell > 72 * 1024) cpb--;
       if constexpr (DIM == 3) {
         const long few = D8 * (S * plane + (long)S * B * B) * nvar;
         // all planes of a cell at once up to ten patches' worth of the chip's
-        // shared memory (order 4: 6,000 cells; beyond, the streamed planes are
-        // level or better)
-        if (!cpb_set && !sel.list && few <= kLimMaxSmem && ncells * few <= 10L * sms * kLimMaxSmem) {
+        // shared memory (five variables, order 4: 6,000 cells; beyond, the
+        // streamed planes are level or better), and fewer where a cell's (plane,
+        // column, variable) items leave three quarters of the CTA idle (order 1,
+        // five variables, 40,000 cells: 45 us, streamed 19; order 2, one variable:
+        // 88 and 28) and at the highest orders (order 6, one variable, 3,000
+        // cells: 95 and 46; order 5, five variables: 81 and 74)
+        const long work = (long)S * B * nvar;
+        long most = 10L * kLimMaxSmem / few;  // cells per SM
+        if (work < 64) most = min(most, max(8L, 7 * work / 10));
+        if (B >= 6) most = min(most, B == 6 ? 12L : 6L);
+        if (!cpb_set && !sel.list && few <= kLimMaxSmem && ncells <= most * sms) {
           cudaError_t e = allow_max_smem(k_lim_to_dg_few<B, NVT>);
           if (e != cudaSuccess) return cuda_status(e, "limiter: shared-memory attribute");
           k_lim_to_dg_few<B, NVT><<<(unsigned)ncells, kLimNT, (size_t)few, st>>>(nvar, ghost, ncells, in, out);
@@ -694,12 +720,14 @@ static exa_status_t lim_run(int op, int nvar, int nobs, int ghost, long ncells, 
     long nblk = (ncells + cpb - 1) / cpb;
     if (sel.count) nblk = nblk < 8L * sms ? nblk : 8L * sms;  // a selection usually holds a few cells: CTAs loop
     if (nblk > 0x7fffffffL) return set_error(EXA_EINVAL, "limiter: too many cells");
-    cudaError_t e = fv ? allow_max_smem(k_lim_to_fv<DIM, B, NVT>) : allow_max_smem(k_lim_to_dg<DIM, B, NVT>);
+    const bool flat = (B <= 2 ? (long)S * S : plane) * nvar < kLimColNT;
+    auto to_dg = flat ? k_lim_to_dg<DIM, B, NVT, true> : k_lim_to_dg<DIM, B, NVT, false>;
+    cudaError_t e = fv ? allow_max_smem(k_lim_to_fv<DIM, B, NVT>) : allow_max_smem(to_dg);
     if (e != cudaSuccess) return cuda_status(e, "limiter: shared-memory attribute");
     if (fv)
       k_lim_to_fv<DIM, B, NVT><<<(unsigned)nblk, nt, smem, st>>>(nvar, ghost, ncells, cpb, in, out, sel);
     else
-      k_lim_to_dg<DIM, B, NVT><<<(unsigned)nblk, kLimColNT, smem, st>>>(nvar, ghost, ncells, cpb, in, out, sel);
+      to_dg<<<(unsigned)nblk, kLimColNT, smem, st>>>(nvar, ghost, ncells, cpb, in, out, sel);
     count_launch();
     return cuda_status(cudaGetLastError(), "limiter projection");
   }
