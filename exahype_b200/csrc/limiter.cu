@@ -12,12 +12,13 @@
 //
 // The reference evaluates every projection as a direct B^dim-term sum per
 // output point.  The operators are tensor products of one 1D table, so here
-// they are applied as dim one-dimensional sums, and a thread keeps all of them
-// for one output column (x, variable) in registers: its x sums from the cell's
-// staged values (loads that the lanes of one variable share, one wavefront
-// each), then y, then z.  No intermediate arrays and no pass over them;
-// consecutive lanes hold consecutive (x, variable), so stores run over whole
-// rows.
+// they are applied as dim one-dimensional sums.  With many columns a thread
+// keeps all of them for one output column (x, variable) in registers: its x sums
+// from the cell's staged values (loads that the lanes of one variable share, one
+// wavefront each), then y, then z.  No intermediate arrays and no pass over
+// them; consecutive lanes hold consecutive (x, variable), so stores run over
+// whole rows.  Few columns take one pass per direction through shared memory
+// (DG -> FV and the extrema), where more threads share a cell.
 //
 // Layouts (the reference's, KernelUtils.h idx4): luh [z][y][x][nvar] with B
 // points per direction; lim [z][y][x][nvar] with S + 2g points per
@@ -99,6 +100,326 @@ __device__ __forceinline__ void lim_stage_cells(double* dst, const double* __res
     for (int i = threadIdx.x; i < nc * n; i += nt) {
       const int c = i / n;
       cp_async8(dst + i, src + sel.cell(c0 + c) * n + (i - c * n));
+    }
+  }
+}
+
+// ------------------------------------------------ few columns: passes
+// The same operators as one pass per direction through shared memory: a
+// column's sums are spread over threads that each own one line, so a cell's
+// chain is short, at the price of a barrier and an intermediate array per pass.
+// Faster than the register columns below while the columns are few (LimPassMax);
+// the sums are the same in the same order, so a cell's values are the same bits.
+
+template <int B>
+struct LimOcc {
+  // resident CTAs per SM the pass kernels are compiled for (register budget of
+  // 64 / 85 / 255 per thread: the least that compiles without spills)
+  static constexpr int value = B <= 4 ? 4 : (B == 5 ? 3 : 1);
+};
+
+// One 1D pass: applies table TAB (NI inputs -> NO outputs, T[p][m]) along
+// direction D of a point array of extents EX x EY x EZ (x fastest), for
+// `ncell` cells and variables v < nv.  Input point p of cell c starts at
+// in + c * cs_in + p * ps_in.  Each thread takes (cell, line, variable)
+// items, the variable fastest, starting with item (threadIdx.x - t0) mod NT
+// (t0 lets a pass continue where the previous pass of the same phase left
+// the threads); it hands the inputs and the NO outputs of its line to
+// out.line<D>(c, x, y, z, v, inputs, outputs, item) with the D coordinate
+// of (x, y, z) 0.  Strides and counts are plain ints: with the variable
+// count a compile-time constant in the caller they fold into immediate
+// offsets.
+template <int TAB, int B, int EX, int EY, int EZ, int D, int NO, class Out>
+__device__ __forceinline__ void lim_pass(const double* in, int ps_in, int cs_in, int ncell, int nv, Out& out,
+                                         int t0 = 0) {
+  constexpr int NI = D == 0 ? EX : (D == 1 ? EY : EZ);
+  constexpr int LINES = EX * EY * EZ / NI;
+  constexpr int SD = D == 0 ? 1 : (D == 1 ? EX : EX * EY);
+  const int items = ncell * LINES * nv;
+  for (int it = (threadIdx.x + kLimNT - t0 % kLimNT) % kLimNT; it < items; it += kLimNT) {
+    const int v = it % nv;
+    const int line = (it / nv) % LINES;
+    const int c = it / (nv * LINES);
+    int x = 0, y = 0, z = 0;
+    if (D == 0) {
+      y = line % EY;
+      z = line / EY;
+    } else if (D == 1) {
+      x = line % EX;
+      z = line / EX;
+    } else {
+      x = line % EX;
+      y = line / EX;
+    }
+    const double* src = in + c * cs_in + ((z * EY + y) * EX + x) * ps_in + v;
+    double a[NI];
+#pragma unroll
+    for (int p = 0; p < NI; p++) a[p] = src[p * SD * ps_in];
+    double o[NO];
+#pragma unroll
+    for (int m = 0; m < NO; m++) {
+      double acc = 0.0;
+#pragma unroll
+      for (int p = 0; p < NI; p++) acc = fma(lim_coef<TAB, B>(p, m), a[p], acc);
+      o[m] = acc;
+    }
+    out.template line<D, NI, NO>(c, x, y, z, v, a, o, it);
+  }
+}
+
+// writes a pass's outputs to a shared-memory array of extents ox x oy x .
+struct SmemOut {
+  double* base;
+  int ps, cs, ox, oy;
+  template <int D, int NI, int NO>
+  __device__ __forceinline__ void line(int c, int x, int y, int z, int v, const double (&)[NI],
+                                       const double (&o)[NO], int) {
+    double* p = base + c * cs + ((z * oy + y) * ox + x) * ps + v;
+    const int st = D == 0 ? ps : (D == 1 ? ox * ps : ox * oy * ps);
+#pragma unroll
+    for (int m = 0; m < NO; m++) p[m * st] = o[m];
+  }
+};
+
+// writes to the interior of ghosted patches
+template <int DIM>
+struct PatchOut {
+  double* base;  // cell 0 of the array
+  long cs;       // doubles per cell
+  int nvar, ext, ghost;
+  long c0;       // first cell of the CTA
+  template <int D, int NI, int NO>
+  __device__ __forceinline__ void line(int c, int x, int y, int z, int v, const double (&)[NI],
+                                       const double (&o)[NO], int) {
+    const long pt = DIM == 3 ? ((long)(z + ghost) * ext + (y + ghost)) * ext + (x + ghost)
+                             : (long)(y + ghost) * ext + (x + ghost);
+    double* p = base + (c0 + c) * cs + pt * nvar + v;
+    const long st = (D == 0 ? 1L : (D == 1 ? (long)ext : (long)ext * ext)) * nvar;
+#pragma unroll
+    for (int m = 0; m < NO; m++) p[m * st] = o[m];
+  }
+};
+
+// extrema of the outputs of a line, stored per item
+struct MinMaxOut {
+  double* pmn;
+  double* pmx;
+  template <int D, int NI, int NO>
+  __device__ __forceinline__ void line(int, int, int, int, int, const double (&)[NI], const double (&o)[NO],
+                                       int it) {
+    double mn = DBL_MAX, mx = -DBL_MAX;
+#pragma unroll
+    for (int m = 0; m < NO; m++) {
+      mn = lim_min(mn, o[m]);
+      mx = lim_max(mx, o[m]);
+    }
+    pmn[it] = mn;
+    pmx[it] = mx;
+  }
+};
+
+// a shared-memory store plus the extrema of the pass's INPUT line (the
+// nodes themselves, seen by the first pass over luh)
+struct SmemOutInputMinMax {
+  SmemOut s;
+  double* pmn;
+  double* pmx;
+  template <int D, int NI, int NO>
+  __device__ __forceinline__ void line(int c, int x, int y, int z, int v, const double (&a)[NI],
+                                       const double (&o)[NO], int it) {
+    s.line<D, NI, NO>(c, x, y, z, v, a, o, it);
+    double mn = DBL_MAX, mx = -DBL_MAX;
+#pragma unroll
+    for (int p = 0; p < NI; p++) {
+      mn = lim_min(mn, a[p]);
+      mx = lim_max(mx, a[p]);
+    }
+    pmn[it] = mn;
+    pmx[it] = mx;
+  }
+};
+
+// shared memory of a cell in k_lim_to_fv_pass (doubles per variable): luh,
+// pass-x and pass-y results (3D)
+template <int DIM, int B>
+__host__ __device__ constexpr int lim_to_fv_pass_doubles() {
+  return DIM == 3 ? B * B * B + B * B * (2 * B - 1) + B * (2 * B - 1) * (2 * B - 1) : B * B + B * (2 * B - 1);
+}
+
+// NVT: the variable count when known at compile time (0 = runtime nvar)
+template <int DIM, int B, int NVT>
+__global__ void __launch_bounds__(kLimNT, LimOcc<B>::value)
+    k_lim_to_fv_pass(int nvar_rt, int ghost, long ncells, int cpb, const double* __restrict__ luh, double* lim) {
+  constexpr int S = 2 * B - 1;
+  constexpr int NPC = DIM == 3 ? B * B * B : B * B;
+  const int nvar = NVT ? NVT : nvar_rt;
+  extern __shared__ double sm[];
+  const long c0 = (long)blockIdx.x * cpb;
+  const int nc = (int)min((long)cpb, ncells - c0);
+  const int SG = S + 2 * ghost;
+  double* A = sm;
+  double* T1 = A + cpb * NPC * nvar;
+  lim_stage_cells(A, luh, NPC * nvar, c0, nc, LimSel(), kLimNT);
+  cp_async_commit_wait_all();
+  __syncthreads();
+  PatchOut<DIM> go{lim, (long)nvar * (DIM == 3 ? SG * SG * SG : SG * SG), nvar, SG, ghost, c0};
+  if (DIM == 2) {
+    SmemOut o1{T1, nvar, S * B * nvar, S, B};
+    lim_pass<kTabUh2Lim, B, B, B, 1, 0, S>(A, nvar, NPC * nvar, nc, nvar, o1);
+    __syncthreads();
+    lim_pass<kTabUh2Lim, B, S, B, 1, 1, S>(T1, nvar, S * B * nvar, nc, nvar, go);
+  } else {
+    double* T2 = T1 + cpb * B * B * S * nvar;
+    SmemOut o1{T1, nvar, B * B * S * nvar, S, B};
+    lim_pass<kTabUh2Lim, B, B, B, B, 0, S>(A, nvar, NPC * nvar, nc, nvar, o1);
+    __syncthreads();
+    SmemOut o2{T2, nvar, B * S * S * nvar, S, S};
+    lim_pass<kTabUh2Lim, B, S, B, B, 1, S>(T1, nvar, B * B * S * nvar, nc, nvar, o2);
+    __syncthreads();
+    lim_pass<kTabUh2Lim, B, S, S, B, 2, S>(T2, nvar, B * S * S * nvar, nc, nvar, go);
+  }
+}
+
+// Extrema and the DMP by passes.  The Gauss-Lobatto (B -> B) and subcell (B -> S) evaluations run side by
+// side, pass by pass; the first pass also takes the extrema of the nodes
+// (its input lines).  Per cell and observable, shared memory holds: the
+// pass-x results of both (B^3 + B^2 S), the pass-y result of the subcells
+// (B S^2) and of the Lobatto points (B^3, in the luh staging area, dead after
+// pass x), and the per-line extrema of nodes, Lobatto points and subcells.
+template <int DIM, int B>
+struct LimMM {
+  static constexpr int S = 2 * B - 1;
+  static constexpr int NPC = DIM == 3 ? B * B * B : B * B;
+  static constexpr int XL = DIM == 3 ? B * B * B : B * B;  // Lobatto pass-x result
+  static constexpr int XS = DIM == 3 ? B * B * S : B * S;  // subcell pass-x result
+  static constexpr int YS = DIM == 3 ? B * S * S : 0;      // subcell pass-y result
+  static constexpr int NODE_LINES = DIM == 3 ? B * B : B;  // pass-x lines
+  static constexpr int LOB_LINES = DIM == 3 ? B * B : B;   // final Lobatto lines
+  static constexpr int SUB_LINES = DIM == 3 ? S * S : S;   // final subcell lines
+  static constexpr int LINES = NODE_LINES + LOB_LINES + SUB_LINES;
+  // doubles per cell
+  __host__ __device__ static constexpr int doubles(int nvar, int nobs) {
+    return NPC * nvar + (XL + XS + YS + 2 * LINES) * nobs;
+  }
+};
+
+// (mode and arguments: k_lim_min_max)
+template <int DIM, int B, int NVT>
+__global__ void __launch_bounds__(kLimNT, LimOcc<B>::value)
+    k_lim_min_max_pass(int mode, int nvar_rt, int nobs_rt, long ncells, int cpb, const double* __restrict__ luh, double relaxation,
+                  double scaling, double* obs_min, double* obs_max, int* dmp_ok) {
+  using M = LimMM<DIM, B>;
+  constexpr int S = M::S, NPC = M::NPC, NF = 2 * DIM;
+  const int nvar = NVT ? NVT : nvar_rt;
+  const int nobs = NVT ? NVT : nobs_rt;
+  extern __shared__ double sm[];
+  const long c0 = (long)blockIdx.x * cpb;
+  const int nc = (int)min((long)cpb, ncells - c0);
+  double* A = sm;                         // luh, later the Lobatto pass-y result
+  double* XL = A + cpb * NPC * nvar;      // [c][z][y][x][obs]
+  double* XS = XL + cpb * M::XL * nobs;
+  double* YS = XS + cpb * M::XS * nobs;
+  double* pmn = YS + cpb * M::YS * nobs;  // [node | lob | sub lines]
+  double* pmx = pmn + cpb * M::LINES * nobs;
+  double* pn_mn = pmn;                    // node lines   [c][line][obs]
+  double* pl_mn = pmn + cpb * M::NODE_LINES * nobs;
+  double* ps_mn = pl_mn + cpb * M::LOB_LINES * nobs;
+  double* pn_mx = pmx;
+  double* pl_mx = pmx + cpb * M::NODE_LINES * nobs;
+  double* ps_mx = pl_mx + cpb * M::LOB_LINES * nobs;
+  if (mode == 1)
+    for (int c = threadIdx.x; c < nc; c += kLimNT) dmp_ok[c0 + c] = 1;
+  lim_stage_cells(A, luh, NPC * nvar, c0, nc, LimSel(), kLimNT);
+  cp_async_commit_wait_all();
+  __syncthreads();
+  const int ix = nc * M::NODE_LINES * nobs;  // items of one pass-x
+  if (DIM == 2) {
+    SmemOutInputMinMax ol{{XL, nobs, B * B * nobs, B, B}, pn_mn, pn_mx};
+    lim_pass<kTabUh2Lob, B, B, B, 1, 0, B>(A, nvar, NPC * nvar, nc, nobs, ol);
+    SmemOut os{XS, nobs, S * B * nobs, S, B};
+    lim_pass<kTabUh2Lim, B, B, B, 1, 0, S>(A, nvar, NPC * nvar, nc, nobs, os, ix);
+    __syncthreads();
+    MinMaxOut ml{pl_mn, pl_mx}, ms{ps_mn, ps_mx};
+    lim_pass<kTabUh2Lob, B, B, B, 1, 1, B>(XL, nobs, B * B * nobs, nc, nobs, ml);
+    lim_pass<kTabUh2Lim, B, S, B, 1, 1, S>(XS, nobs, S * B * nobs, nc, nobs, ms, nc * B * nobs);
+  } else {
+    SmemOutInputMinMax ol{{XL, nobs, B * B * B * nobs, B, B}, pn_mn, pn_mx};
+    lim_pass<kTabUh2Lob, B, B, B, B, 0, B>(A, nvar, NPC * nvar, nc, nobs, ol);
+    SmemOut os{XS, nobs, B * B * S * nobs, S, B};
+    lim_pass<kTabUh2Lim, B, B, B, B, 0, S>(A, nvar, NPC * nvar, nc, nobs, os, ix);
+    __syncthreads();
+    double* YL = A;  // luh is dead after pass x
+    SmemOut yl{YL, nobs, B * B * B * nobs, B, B};
+    lim_pass<kTabUh2Lob, B, B, B, B, 1, B>(XL, nobs, B * B * B * nobs, nc, nobs, yl);
+    SmemOut ys{YS, nobs, B * S * S * nobs, S, S};
+    lim_pass<kTabUh2Lim, B, S, B, B, 1, S>(XS, nobs, B * B * S * nobs, nc, nobs, ys, nc * B * B * nobs);
+    __syncthreads();
+    MinMaxOut ml{pl_mn, pl_mx}, ms{ps_mn, ps_mx};
+    lim_pass<kTabUh2Lob, B, B, B, B, 2, B>(YL, nobs, B * B * B * nobs, nc, nobs, ml);
+    lim_pass<kTabUh2Lim, B, S, S, B, 2, S>(YS, nobs, B * S * S * nobs, nc, nobs, ms, nc * B * B * nobs);
+  }
+  __syncthreads();
+  // per (cell, observable): the new extrema -> face blocks, and the DMP
+  auto finish = [&](int pair, double mn, double mx) {
+    const int c = pair / nobs, v = pair % nobs;
+    double* bmn = obs_min + (c0 + c) * NF * nobs;
+    double* bmx = obs_max + (c0 + c) * NF * nobs;
+    if (mode == 0) {
+      for (int f = 0; f < NF; f++) {
+        bmn[f * nobs + v] = mn;
+        bmx[f * nobs + v] = mx;
+      }
+    } else {
+      double lo = bmn[v], hi = bmx[v];
+      for (int f = 1; f < NF; f++) {
+        lo = lim_min(lo, bmn[f * nobs + v]);
+        hi = lim_max(hi, bmx[f * nobs + v]);
+      }
+      const double sd = lim_max((hi - lo) * scaling, relaxation);
+      if (mn < lo - sd || mx > hi + sd) atomicAnd(dmp_ok + c0 + c, 0);
+      bmn[v] = mn;
+      bmx[v] = mx;
+      bmn[v + nobs] = lo;
+      bmx[v + nobs] = hi;
+    }
+  };
+  auto line_index = [&](int c, int v, int l) {
+    if (l < M::NODE_LINES) return (c * M::NODE_LINES + l) * nobs + v;
+    if (l < M::NODE_LINES + M::LOB_LINES)
+      return cpb * M::NODE_LINES * nobs + (c * M::LOB_LINES + l - M::NODE_LINES) * nobs + v;
+    return cpb * (M::NODE_LINES + M::LOB_LINES) * nobs + (c * M::SUB_LINES + l - M::NODE_LINES - M::LOB_LINES) * nobs +
+           v;
+  };
+  // reduction over the line extrema: a thread per pair when the pairs have
+  // few lines (2D), a warp per pair otherwise
+  if (M::LINES <= 32) {
+    for (int pair = threadIdx.x; pair < nc * nobs; pair += kLimNT) {
+      const int c = pair / nobs, v = pair % nobs;
+      double mn = DBL_MAX, mx = -DBL_MAX;
+#pragma unroll
+      for (int l = 0; l < M::LINES; l++) {
+        const int k = line_index(c, v, l);
+        mn = lim_min(mn, pmn[k]);
+        mx = lim_max(mx, pmx[k]);
+      }
+      finish(pair, mn, mx);
+    }
+  } else {
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    for (int pair = warp; pair < nc * nobs; pair += kLimNT / 32) {
+      const int c = pair / nobs, v = pair % nobs;
+      double mn = DBL_MAX, mx = -DBL_MAX;
+      for (int l = lane; l < M::LINES; l += 32) {
+        const int k = line_index(c, v, l);
+        mn = lim_min(mn, pmn[k]);
+        mx = lim_max(mx, pmx[k]);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        mn = lim_min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        mx = lim_max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      }
+      if (lane == 0) finish(pair, mn, mx);
     }
   }
 }
@@ -621,17 +942,57 @@ __global__ void __launch_bounds__(kLimNT) k_lim_fv_min_max(int nvar, int nobs, i
   }
 }
 
+// Columns (subcell columns x variables; for the extrema subcell and Lobatto
+// columns x observables) of a call up to which it takes the passes, by B: the
+// largest calls that measured faster there.  With five variables / observables
+// and with any other number.  us per call, passes and columns: one 3D cell of
+// order 4, DG -> FV 3.8 / 4.7, DMP 4.8 / 6.2, of order 6 7.8 / 9.4 and 8.4 / 11.3,
+// one 2D cell of order 3 2.4 / 3.3 and 3.1 / 4.3; 100 3D cells of order 5, DMP
+// 6.3 / 8.8; 5,000 2D cells of order 4, DMP 7.1 / 9.0; 300 3D cells of order 6
+// with one variable, DG -> FV 7.9 / 19, extrema 8.9 / 23.
+template <int DIM, bool FIVE>
+struct LimPassMax {
+  static constexpr long fv2[2][8] = {{0, 0, 90, 135, 1008000, 180, 198, 156}, {0, 0, 150, 250, 700000, 135, 165, 65}};
+  static constexpr long fv3[2][8] = {{0, 0, 0, 30, 63, 360000, 44, 11700}, {0, 0, 45, 25, 28000, 45, 5500, 6500}};
+  static constexpr long mm2[2][8] = {{0, 0, 0, 216, 13200, 280, 306, 240}, {0, 0, 0, 400, 110000, 840000, 255, 300}};
+  static constexpr long mm3[2][8] = {{0, 0, 0, 0, 66, 11200, 13600, 320000}, {0, 0, 0, 40, 55, 84000, 102000, 30000}};
+  static constexpr long fv(int B) { return DIM == 2 ? fv2[FIVE][B] : fv3[FIVE][B]; }
+  static constexpr long mm(int B) { return DIM == 2 ? mm2[FIVE][B] : mm3[FIVE][B]; }
+};
+
+// cells per CTA of the passes: enough items for two rounds of the final pass,
+// within a shared-memory budget that leaves room for `occ` resident CTAs per SM
+static int lim_pass_cpb(long items_per_cell, long smem_per_cell, long ncells, int occ) {
+  long cpb = (2 * kLimNT + items_per_cell - 1) / items_per_cell;
+  const long cap = (220L * 1024 / occ) / smem_per_cell;
+  cpb = min(cpb, min(64L, min(cap, ncells)));
+  return (int)(cpb < 1 ? 1 : cpb);
+}
+
 // cells per CTA: the count whose items fill their rounds of nt threads best,
 // within a shared-memory budget and up to 16 or one round's cells; no more than
-// leave every SM four CTAs
-static int lim_cpb(long items_per_cell, long smem_per_cell, long ncells, int nt, long budget, int sms) {
+// leave every SM four CTAs, but at least what lets all CTAs be resident at once
+// (`occ` per SM) where that takes a few cells and no further round or, for the
+// extrema, saves a wave that would be nearly empty: 1,200 3D cells of order 6, one
+// observable, 17.5 us with six cells per CTA, 36 with one; 1,200 2D cells of
+// order 5 5.5 and 7.0.  `latency`: share of a round that a CTA waits before its
+// first one; more rounds share it (extrema of 12,000 2D cells of order 6, three
+// observables: 23 us with eight cells, 28 with two).
+static int lim_cpb(long items_per_cell, long smem_per_cell, long ncells, int nt, long budget, int sms, int occ,
+                   bool extrema, double latency) {
   int best = 1;
   double fill = 0.0;
   const long round = nt / items_per_cell, most = round > 16 ? round : 16, spread = ncells / (4 * sms);
   for (int c = 1; c <= most && (c == 1 || (c * smem_per_cell <= budget && c <= spread)); c++) {
-    const long items = c * items_per_cell;
-    const double f = (double)items / (double)((items + nt - 1) / nt * nt);
+    const long items = c * items_per_cell, rounds = (items + nt - 1) / nt;
+    const double f = (double)items / (double)(rounds * nt) * (1.0 - latency / (double)rounds);
     if (f > fill + 0.02) best = c, fill = f;
+  }
+  const long slots = (long)occ * sms, once = (ncells + slots - 1) / slots;
+  if (once > best && once <= 8 && once * smem_per_cell * occ <= 220L * 1024) {
+    const long rounds = (once * items_per_cell + nt - 1) / nt, rounds1 = (items_per_cell + nt - 1) / nt;
+    if (rounds <= rounds1 || (extrema && rounds <= once * rounds1 && 2 * once * slots > 3 * ncells))
+      best = (int)once;
   }
   return best;
 }
@@ -645,8 +1006,7 @@ static exa_status_t lim_run(int op, int nvar, int nobs, int ghost, long ncells, 
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // The entry points take cells whose 1D passes' arrays fit one CTA's shared
-  // memory (doubles per variable or observable below); the column kernels need
-  // none, the limit stands.
+  // memory (doubles per variable or observable below).
   constexpr long P = DIM == 3 ? B * B * B : B * B, Q = DIM == 3 ? S * S * S : S * S;
   constexpr long fv_pass = DIM == 3 ? P + B * B * S + B * S * S : P + B * S;
   constexpr long dg_pass = DIM == 3 ? Q + S * S * B : Q + S * B;
@@ -659,6 +1019,24 @@ static exa_status_t lim_run(int op, int nvar, int nobs, int ghost, long ncells, 
     return set_error(EXA_EINVAL, "limiter: cell too large for shared memory");
   constexpr long NPC = P, D8 = (long)sizeof(double);
   const int cpb_set = tune_get(kTuneLimiterCellsPerCta, 0);
+  const bool mm = op == kLimMinMax || op == kLimDmp;
+  if ((op == kLimToFv && !sel.list && ncells * S * nvar <= LimPassMax<DIM, NVT == 5>::fv(B)) ||
+      (mm && ncells * COLS * nobs <= LimPassMax<DIM, NVT == 5>::mm(B))) {
+    const long lines = DIM == 3 ? S * S : S;  // of the final pass
+    const long per_cell = D8 * (mm ? LimMM<DIM, B>::doubles(nvar, nobs) : lim_to_fv_pass_doubles<DIM, B>() * nvar);
+    int cpb = lim_pass_cpb(lines * (mm ? nobs : nvar), per_cell, ncells, LimOcc<B>::value);
+    if (cpb_set > 0 && (long)cpb_set * per_cell <= kLimMaxSmem) cpb = cpb_set;
+    const unsigned nblk = (unsigned)((ncells + cpb - 1) / cpb);
+    cudaError_t e = mm ? allow_max_smem(k_lim_min_max_pass<DIM, B, NVT>) : allow_max_smem(k_lim_to_fv_pass<DIM, B, NVT>);
+    if (e != cudaSuccess) return cuda_status(e, "limiter: shared-memory attribute");
+    if (mm)
+      k_lim_min_max_pass<DIM, B, NVT><<<nblk, kLimNT, (size_t)cpb * per_cell, st>>>(
+          op == kLimDmp ? 1 : 0, nvar, nobs, ncells, cpb, in, relax, scaling, mn, mx, ok);
+    else
+      k_lim_to_fv_pass<DIM, B, NVT><<<nblk, kLimNT, (size_t)cpb * per_cell, st>>>(nvar, ghost, ncells, cpb, in, out);
+    count_launch();
+    return cuda_status(cudaGetLastError(), "limiter pass kernel");
+  }
   if (op == kLimToFv || op == kLimToDg) {
     const bool fv = op == kLimToFv;
     // one column per thread of the last cell's end at most: FV -> DG walks its
@@ -669,7 +1047,7 @@ static exa_status_t lim_run(int op, int nvar, int nobs, int ghost, long ncells, 
     int cpb;
     int nt = kLimColNT;
     if (fv) {
-      cpb = lim_cpb(items, per_cell, ncells, kLimColNT, 44 * 1024, sms);
+      cpb = lim_cpb(items, per_cell, ncells, kLimColNT, 44 * 1024, sms, LimMinB<DIM, B, true>::value, false, 0.0);
       if (DIM == 3) {
         // one round of columns if they fill whole warps well (order 4, 24,000
         // cells: 313 us, three rounds 348; order 6, a third of its lanes idle:
@@ -740,13 +1118,15 @@ static exa_status_t lim_run(int op, int nvar, int nobs, int ghost, long ncells, 
   const bool walk = DIM == 2 && (B <= 4 || (B <= 6 && ncells * nobs >= 512L * sms));
   if (op == kLimFvMinMax) {
     per_cell = (long)(DIM == 3 ? S * S * S : S * S) * nvar * (long)sizeof(double);
-    // a warp per (cell, observable), two rounds of them, three CTAs per SM
-    const long want = (16 + nobs - 1) / nobs, cap = 73L * 1024 / per_cell;
+    // a warp per (cell, observable), two rounds of them, three CTAs per SM (four
+    // up to order 3: 100 3D cells with five of twelve variables 8 us, 13 with three)
+    const long want = (16 + nobs - 1) / nobs, cap = (B <= 4 ? 55L : 73L) * 1024 / per_cell;
     cpb = (int)(want < cap ? want : (cap < 1 ? 1 : cap));
     if (cpb > ncells) cpb = (int)ncells;
   } else {
     per_cell = D8 * (walk ? lim_pitch<DIM, B, true>(nvar) : NPC * nvar + 2L * COLS * nobs);
-    cpb = lim_cpb((walk ? 1L : (long)COLS) * nobs, per_cell, ncells, kLimMmNT, 36 * 1024, sms);
+    cpb = lim_cpb((walk ? 1L : (long)COLS) * nobs, per_cell, ncells, kLimMmNT, 36 * 1024, sms,
+                  walk ? LimMmMinB<DIM, B, true>::value : LimMmMinB<DIM, B, false>::value, true, NVT ? 0.0 : 0.25);
   }
   if (cpb_set > 0 && (long)cpb_set * per_cell <= kLimMaxSmem) cpb = cpb_set;
   const size_t smem = (size_t)cpb * per_cell;
