@@ -26,13 +26,16 @@ def _time_ensemble(ens, steps):
     return t.elapsed_ms() / steps
 
 
-def tune_contraction(ens, steps=3, mask=0x30):
+def tune_contraction(ens, steps=3, mask=None):
     """Coordinate descent over the contraction of each order present
     (pencil or line-owner against node-gather; exa_ensemble_tune_contraction)
-    in the ensemble's current launch form and schedule, from `mask` (the
-    library's defaults: 0x3c in FP64, 0x30 mixed), flipping one order at a time and
-    keeping the faster.  Applies the result and returns (mask, table)."""
+    in the ensemble's current launch form and schedule, from `mask` (default: the
+    one in force, which for a new ensemble is the library's: 0x3c in FP64, 0x30
+    mixed), flipping one order at a time and keeping the faster.  Applies the
+    result and returns (mask, table); orders that are not present keep their bit."""
     table = []
+    if mask is None:
+        mask = ens.lines_mask
     present = sorted({c.order for c in ens.cfgs.values()})
     if not present:
         return mask, table
@@ -78,10 +81,9 @@ def tune_ensemble(ens, steps=3, ctas=(1, 2), grabs=(1, 2, 4, 8), orders=(0, 1), 
             ens.set_launch_mode(lm)
             return tuple(got['best']), got['table']
     table = []
-    mask = 0x30  # start of the descent: orders 4 and 5
     if contraction and ens.cfgs:
         ens.tune(ctas[0], grabs[0], orders[0])
-        mask, table = tune_contraction(ens, steps, mask)
+        _, table = tune_contraction(ens, steps)
     for c, g, o in itertools.product(ctas, grabs, orders):
         ens.tune(c, g, o)
         ms = _time_ensemble(ens, steps)
@@ -95,7 +97,7 @@ def tune_ensemble(ens, steps=3, ctas=(1, 2), grabs=(1, 2, 4, 8), orders=(0, 1), 
         table.append({'stage': 'launch_mode', 'launch_mode': 1, 'ms_per_step': ms})
         mode = 1 if (ms < best['ms_per_step'] or 0 not in modes) else 0
     ens.set_launch_mode(mode)
-    b = (best['ctas_per_sm'], best['grab'], best['order_policy'], mask, mode)
+    b = (best['ctas_per_sm'], best['grab'], best['order_policy'], ens.lines_mask, mode)
     if cache and key:
         data = {}
         if os.path.exists(cache):

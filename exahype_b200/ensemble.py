@@ -42,6 +42,8 @@ class Ensemble:
         self.h = h
         self.max_solves = max_solves
         self.cfgs = {}
+        # contraction per order in force (tune_contraction): the library's default
+        self.lines_mask = 0x30 if precision == _lib.PREC_MIXED else 0x3c
 
     def add(self, cfg, steps=-1):
         """Admits a solve; returns its slot, or None when it does not fit now."""
@@ -70,6 +72,7 @@ class Ensemble:
         """Per order N: bit N set = pencil (FP64) or line-owner (mixed)
         contraction, clear = node-gather."""
         call('exa_ensemble_tune_contraction', self.h, int(lines_mask))
+        self.lines_mask = int(lines_mask)
 
     def set_launch_mode(self, mode):
         """0: one persistent launch per step; 1: one launch per order and phase."""
