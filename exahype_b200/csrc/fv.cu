@@ -103,9 +103,9 @@ __device__ __forceinline__ long fv_stencil_offset(const FVArgs& a, int X, int Y,
 
 
 // Pressure, sound speed, flux and largest |eigenvalue| of a cell for the Godunov
-// kernels, with every multiply-add written out: a sum of two products may be
-// fused either way round, and the sweeps and the tile kernel are to give the
-// same bits.
+// kernels, with every multiply-add written out, as in their updates: a sum of two
+// products may be fused either way round, and the sweeps and the tile kernel are
+// to give the same bits.
 template <bool PLANAR>
 struct FVPoint {
   double irho, p, c;
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(32 * FVS_WARPS) k_fv_godunov_sweep(FVArgs a) {
 #pragma unroll
       for (int m = 0; m < V; m++) {
         v[m] = part[m];
-        v[m] -= cy * fy[m];
+        v[m] = fma(-cy, fy[m], v[m]);
       }
       double* o = a.out + (rc_up + colc) * D;  // row r - 1, in the domain
 #pragma unroll
@@ -336,9 +336,9 @@ __global__ void __launch_bounds__(32 * FVS_WARPS) k_fv_godunov_sweep(FVArgs a) {
 #pragma unroll
     for (int m = 0; m < V; m++) {
       double v = u[m];
-      v += cx * fxl[m];
-      v -= cx * fxr[m];
-      v += cy * fy[m];
+      v = fma(cx, fxl[m], v);
+      v = fma(-cx, fxr[m], v);
+      v = fma(cy, fy[m], v);
       part[m] = v;
     }
 #pragma unroll
@@ -456,17 +456,17 @@ __global__ void __launch_bounds__(32 * FVS_WARPS) k_fv_godunov_batch(FVArgs a, F
       if (j > j0) {
         double* d = o + (j - 1) * row;
 #pragma unroll
-        for (int m = 0; m < V; m++) d[m] = part[m] - cy * fy[m];
+        for (int m = 0; m < V; m++) d[m] = fma(-cy, fy[m], part[m]);
       }
       if (j == pb) {
         double* d = o + (pb - 1) * row;
 #pragma unroll
-        for (int m = 0; m < V; m++) d[m] -= cy * fy[m];
+        for (int m = 0; m < V; m++) d[m] = fma(-cy, fy[m], d[m]);
       }
       if (j == pe) {
         double* d = o + pe * row;
 #pragma unroll
-        for (int m = 0; m < V; m++) d[m] += cy * fy[m];
+        for (int m = 0; m < V; m++) d[m] = fma(cy, fy[m], d[m]);
       }
     }
     if (j == j1) break;
@@ -486,17 +486,17 @@ __global__ void __launch_bounds__(32 * FVS_WARPS) k_fv_godunov_batch(FVArgs a, F
     if (inside) {
 #pragma unroll
       for (int m = 0; m < V; m++) {
-        v[m] += cx * fxl[m];
-        v[m] -= cx * fxr[m];
-        v[m] += cy * fy[m];
+        v[m] = fma(cx, fxl[m], v[m]);
+        v[m] = fma(-cx, fxr[m], v[m]);
+        v[m] = fma(cy, fy[m], v[m]);
         part[m] = v[m];
       }
     } else if (left_ghost) {
 #pragma unroll
-      for (int m = 0; m < V; m++) o[j * row + m] = v[m] - cx * fxr[m];
+      for (int m = 0; m < V; m++) o[j * row + m] = fma(-cx, fxr[m], v[m]);
     } else if (right_ghost) {
 #pragma unroll
-      for (int m = 0; m < V; m++) o[j * row + m] = v[m] + cx * fxl[m];
+      for (int m = 0; m < V; m++) o[j * row + m] = fma(cx, fxl[m], v[m]);
     }
     // every face of the strip: the left one of each interior cell and, from
     // the lane right of it, the right one of the strip's last cell
@@ -592,10 +592,10 @@ __device__ __forceinline__ void fv_godunov_tile(const FVArgs& a, int bx, int by)
 #pragma unroll
     for (int m = 0; m < V; m++) {
       double u = q[m];
-      u += cx * fxl[m];
-      u -= cx * fxr[m];
-      u += cy * fyb[m];
-      u -= cy * fyt[m];
+      u = fma(cx, fxl[m], u);
+      u = fma(-cx, fxr[m], u);
+      u = fma(cy, fyb[m], u);
+      u = fma(-cy, fyt[m], u);
       o[m] = u;
       un[m] = u;
     }
