@@ -167,12 +167,14 @@ static exa_status_t launch_dn(const exa_aderdg_desc_t& d, const PredArgs& a, int
   // line-owner): 2D orders 2..5 309 / 478, 398 / 524, 544 / 721, 578 / 845
   // (156,000 to 27,641 cells), 3D orders 3..5 1648 / 2253, 3337 / 4073,
   // 2371 / 2823 (82,000, 68,921 and 15,000 cells).  In 3D order 2 (27 threads
-  // a cell, 45 T tasks on them) it measured 1794 against 1757 for line-owner.
+  // a cell, 45 T tasks on them) it measured 1794 against 1757 for line-owner, which
+  // runs there at every size (node-gather: 11.5 / 12.6 us up to 100 cells, 15.2 /
+  // 16.3 at 1000, 42.0 / 40.1 at 3000, 1073 / 1005 at 100,000).
   // Few 2D cells of orders 2 and 5: the line-owner form while one wave of it
   // holds them.  It spreads a cell's work over more threads, whose chain is all
-  // that counts there: order 5 18.4 / 24.6 us at 24 cells, 20.7 / 24.6 at 576,
-  // but 38.9 / 27.0 at 625 (four CTAs of a cell per SM); order 2 10.2 / 11.3 us
-  // at 400 to 1156 cells, level at 2025.
+  // that counts there: order 5 26.6 / 34.6 us at 24 cells, 29.6 / 35.6 at 576,
+  // but 52.8 / 35.7 at 625 (four CTAs of a cell per SM); order 2 8.6 / 9.9 us at
+  // 24 cells, 8.8 / 10.3 at 1150, level at 1300 to 2000, 12.7 / 12.3 at 3000.
   // Both forms give a cell the same bits, so that neither the cells beside it in
   // a call nor the cut of a grid into slabs shows in its values.
   // knob 3 selects another: 1 = node-gather, 2 = line-owner contraction, 3 =

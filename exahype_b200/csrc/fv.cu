@@ -195,10 +195,6 @@ __device__ __forceinline__ double fv_face_flux(const double* qL, const double* q
   return smax;
 }
 
-// five 256-thread CTAs (42 KB each) per SM: 48 registers and the largest
-// shared-memory carveout
-// One FV_TX x FV_TY tile (tile column bx, row by) of patch `patch` of a.luh
-// / a.out (the body of k_fv_godunov; the serving batch calls it per entry).
 // Godunov step as a sweep in y (one periodic patch, or the global view of a
 // patch grid): each warp owns a strip of FVS_W output columns (lane l =
 // column k0 - 1 + l; lanes 0 and 31 are halo columns) and walks up a.rows
@@ -542,6 +538,8 @@ __global__ void k_fv_inf(unsigned long long* slots, long n) {
   if (i < n) slots[i] = 0x7FF0000000000000ULL;
 }
 
+// One FV_TX x FV_TY tile (tile column bx, row by) of a.luh / a.out (the body of
+// k_fv_godunov; the serving batch calls it per entry)
 template <bool PLANAR, bool GRID = false>
 __device__ __forceinline__ void fv_godunov_tile(const FVArgs& a, int bx, int by) {
   constexpr int V = kV, C = kV + 1;
@@ -604,6 +602,8 @@ __device__ __forceinline__ void fv_godunov_tile(const FVArgs& a, int bx, int by)
   ndt.commit(a, a.next_dt, (tid & 31) == 0);
 }
 
+// five 256-thread CTAs (42 KB each) per SM: 48 registers and the largest
+// shared-memory carveout
 template <bool PLANAR, bool GRID = false>
 __global__ void __launch_bounds__(FV_NT, 5) k_fv_godunov(FVArgs a) {
   fv_godunov_tile<PLANAR, GRID>(a, blockIdx.x, blockIdx.y);
