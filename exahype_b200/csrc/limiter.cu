@@ -1020,8 +1020,12 @@ static exa_status_t lim_run(int op, int nvar, int nobs, int ghost, long ncells, 
   constexpr long NPC = P, D8 = (long)sizeof(double);
   const int cpb_set = tune_get(kTuneLimiterCellsPerCta, 0);
   const bool mm = op == kLimMinMax || op == kLimDmp;
+  // (3D calls whose columns just fill one wave, one cell per CTA, are level with
+  // the passes and ahead of them when their cells are not in L2)
+  const long wave = (long)LimMmMinB<DIM, B, false>::value * sms;
+  const bool full_wave = DIM == 3 && ncells <= wave && 20 * ncells > 17 * wave;
   if ((op == kLimToFv && !sel.list && ncells * S * nvar <= LimPassMax<DIM, NVT == 5>::fv(B)) ||
-      (mm && ncells * COLS * nobs <= LimPassMax<DIM, NVT == 5>::mm(B))) {
+      (mm && !full_wave && ncells * COLS * nobs <= LimPassMax<DIM, NVT == 5>::mm(B))) {
     const long lines = DIM == 3 ? S * S : S;  // of the final pass
     const long per_cell = D8 * (mm ? LimMM<DIM, B>::doubles(nvar, nobs) : lim_to_fv_pass_doubles<DIM, B>() * nvar);
     int cpb = lim_pass_cpb(lines * (mm ? nobs : nvar), per_cell, ncells, LimOcc<B>::value);
