@@ -368,7 +368,9 @@ struct FVStrips {
   int rows;      // rows of a block
 };
 
-static FVStrips fv_strips(int P, long npatches) {
+// in_place: luh_new is luh.  A patch of one strip and one block of rows reads
+// every cell before it writes it; blocks would read their neighbour's new rows.
+static FVStrips fv_strips(int P, long npatches, bool in_place) {
   FVStrips s;
   s.width = P < 30 ? P : 30;
   s.per_warp = 32 / (s.width + 2);
@@ -391,7 +393,7 @@ static FVStrips fv_strips(int P, long npatches) {
   };
   auto cost = [](int h, long n) { return (h + 2) * (2 * n > 5 ? 2 * n : 5); };
   long least = cost(top, ctas(top, s.per_warp));
-  if (ctas(top, s.per_warp) <= 4)
+  if (ctas(top, s.per_warp) <= 4 && !in_place)
     for (int h = top - 1; h >= 1; h--) {
       const long c = cost(h, ctas(h, 1));
       if (c < least) s.rows = h, least = c;
@@ -1424,7 +1426,7 @@ static exa_status_t fv_update(int scheme, const exa_fv_desc_t* desc, long npatch
   a.max_dt = (unsigned long long*)max_dt;
   const bool planar = desc->pde == EXA_PDE_EULER_PLANAR;
   if (scheme == 0) {
-    const FVStrips s = fv_strips(desc->patch, npatches);
+    const FVStrips s = fv_strips(desc->patch, npatches, luh_new == luh);
     if (s.across * s.up > 1)
       if (exa_status_t e = clear_max_dt()) return e;
     const long warps = (s.units + s.per_warp - 1) / s.per_warp;
